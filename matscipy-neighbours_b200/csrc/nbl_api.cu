@@ -567,6 +567,7 @@ static void traverse_args(Plan &p, const Batch &b) {
     ta.pos32 = B.pos32;
     ta.aux = B.aux;
     ta.amax = B.amax;
+    ta.per_atom = B.per_atom;
     ta.pt32 = B.pt32;
     ta.pt64 = B.pt64;
     ta.counts = B.counts;

@@ -61,6 +61,7 @@ struct TraverseArgs {
     const float4 *pos32;
     const int4 *aux;
     const float *amax;
+    const double *per_atom;   // [natoms] per-atom radii (original order) or null
     const float *pt32;        // per-type squared cutoffs, FP32
     const double *pt64;       // per-type squared cutoffs, FP64
     int64_t natoms;           // atoms of the batch (offsets[natoms] = pair total)

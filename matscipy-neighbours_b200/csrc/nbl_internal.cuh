@@ -9,8 +9,9 @@
 //                       (dense: indexed by cell_base + linear cell; hashed:
 //                       indexed by hash slot)
 //   hkey[cap]           hashed grid only: composite (system, linear cell) key
-//   pos64[N]  double4   cell-sorted bin-relative position (x, y, z) and the
-//                       per-atom cutoff radius (w) -- the FP64 operands
+//   pos64[N]  double4   cell-sorted bin-relative position (x, y, z), the FP64
+//                       operands, and in the bits of w the global atom index
+//                       (low word) and the packed image index (high word)
 //   pos32[N]  float4    the same position rounded to FP32 (x, y, z) and the
 //                       per-atom radius (FP32) or the type id (int bits) (w)
 //   aux[N]    int4      (global atom index, q0, q1, q2): q is the atom's
@@ -154,6 +155,20 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
 __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_all;\n" ::: "memory");
 }
+
+// Packed image indices: three signed fields as one sum, so that differences
+// of packed values are packed differences.  With every |q| <= 127 a sum of
+// three such values stays inside its 10-bit field; others are kImageWide and
+// read from the full records instead.
+constexpr int kImageWide = INT32_MIN;
+__host__ __device__ __forceinline__ int pack_image(int q0, int q1, int q2) {
+    const bool in = q0 >= -127 && q0 <= 127 && q1 >= -127 && q1 <= 127 && q2 >= -127 &&
+                    q2 <= 127;
+    return in ? q0 + q1 * 1024 + q2 * (1024 * 1024) : kImageWide;
+}
+// Added to a packed value: every field non-negative, field k's value at bits
+// 10 k is ((v >> 10 k) & 1023) - 512.
+constexpr int kImageBias = 512 + 512 * 1024 + 512 * 1024 * 1024;
 
 // Kernel launches issued by the calling host thread (reported through
 // nbl_launch_count()); every launch site bumps it.

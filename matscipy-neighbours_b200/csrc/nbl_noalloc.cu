@@ -278,6 +278,7 @@ extern "C" NBL_API nbl_status nbl_neighbour_list_noalloc(const nbl_request *req,
     ta.pos32 = pos32;
     ta.aux = aux;
     ta.amax = amax;
+    ta.per_atom = per_atom;
     ta.pt32 = pt32;
     ta.pt64 = pt64;
     ta.counts = counts;

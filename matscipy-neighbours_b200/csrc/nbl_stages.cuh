@@ -115,15 +115,18 @@ __device__ __forceinline__ void gather_one(const GatherArgs &a, int64_t s) {
             v = dsub(v, dmul((double)rc[2], S.bin[2][k]));
             rel[k] = v;
         }
-        double w64 = 0.0;
         float w32 = 0.f;
         if (S.cutoff_kind == kCutPerAtom) {
-            w64 = a.per_atom[at];
-            w32 = __double2float_rn(w64);
+            w32 = __double2float_rn(a.per_atom[at]);
         } else if (S.cutoff_kind == kCutPerType) {
             w32 = __int_as_float(a.types[at]);
         }
-        a.pos64[s] = make_double4(rel[0], rel[1], rel[2], w64);
+        // the image index packs unless it is large, or is an open axis' quirk
+        // (which the pair's j side must not contribute)
+        const bool quirk = (!S.pbc[0] && q[0] != 0) || (!S.pbc[1] && q[1] != 0) ||
+                           (!S.pbc[2] && q[2] != 0);
+        const int qp = quirk ? kImageWide : pack_image(q[0], q[1], q[2]);
+        a.pos64[s] = make_double4(rel[0], rel[1], rel[2], __hiloint2double(qp, at));
         a.pos32[s] = make_float4(__double2float_rn(rel[0]), __double2float_rn(rel[1]),
                                  __double2float_rn(rel[2]), w32);
         a.aux[s] = make_int4(at, q[0], q[1], q[2]);
