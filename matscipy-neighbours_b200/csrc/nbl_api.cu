@@ -229,6 +229,57 @@ static int64_t mask_words(const Plan &p, const Batch &b) {
     return (int64_t)w;
 }
 
+// Expected neighbours per atom of system s at uniform density.
+static double expected_row(const Batch &b, size_t s) {
+    const SysDev &S = b.sys[s];
+    const double(*c)[3] = S.bin;
+    const double cell = std::fabs(c[0][0] * (c[1][1] * c[2][2] - c[1][2] * c[2][1]) -
+                                  c[0][1] * (c[1][0] * c[2][2] - c[1][2] * c[2][0]) +
+                                  c[0][2] * (c[1][0] * c[2][1] - c[1][1] * c[2][0]));
+    const double vol = cell * (double)std::max<int64_t>(b.ncells[s], 1);
+    return (double)S.nat * 4.18879 * S.cutoff * S.cutoff * S.cutoff / std::max(vol, 1e-300);
+}
+
+// Entries per atom for a mean row of m: room for a uniform system's scatter
+// (longer rows chain on).
+static double list_entries(double m) { return 1.1 * m + 4.0 * std::sqrt(m) + 4.0; }
+
+// Sizes of the neighbour lists: every system's entries per atom follow its
+// density, scaled by what the last count of the same sizes found (surfaces,
+// cutoffs below the widest); a quarter on top, or what the last count took
+// and more, for chained chunks.
+static ListPlan plan_lists(const Plan &p, const Batch &b) {
+    ListPlan lp;
+    const bool known = p.list_natoms == b.natoms && p.list_table == b.table_size;
+    const double scale = known ? p.list_scale : 1.0;
+    int max_visit = 0;
+    for (const SysDev &S : b.sys) max_visit = std::max(max_visit, S.nvisit);
+    lp.shift = 32 - bits_for((uint64_t)std::max(max_visit - 1, 1));
+    lp.wide = b.natoms > (int64_t(1) << lp.shift);
+    double own = 0.0, mean = 0.0;
+    for (size_t s = 0; s < b.sys.size(); s++) {
+        const double m = expected_row(b, s);
+        mean += m * (double)b.sys[s].nat;
+        own += list_entries(std::min(scale * m, 1e6)) * (double)b.sys[s].nat;
+    }
+    lp.expect = mean;
+    lp.scale = scale;
+    // at most 2^30 entries up front
+    lp.shrink = own > (double)(int64_t(1) << 30) ? (double)(int64_t(1) << 30) / own : 1.0;
+    int64_t at = 0;
+    for (size_t s = 0; s < b.sys.size(); s++) at += lp.cap(expected_row(b, s)) * b.sys[s].nat;
+    lp.chunks = at;
+    const int64_t more = std::max<int64_t>(
+        std::max<int64_t>(at / 4, known ? p.list_hint + p.list_hint / 4 : 0), int64_t(1) << 16);
+    lp.total = at + more;
+    lp.row_cap = known && b.natoms > kMarkAtoms ? lp.total * 4 / kRowChunk + 16 : 0;
+    return lp;
+}
+int64_t ListPlan::cap(double m) const {
+    const double e = list_entries(std::min(scale * m, 1e6)) * shrink;
+    return (int64_t)std::ceil(e / (wide ? 2.0 : 4.0)) + 1;  // and the link
+}
+
 // Carve the per-call buffers out of the plan's workspace.
 static nbl_status layout_workspace(Plan &p, const Batch &b) {
     const int64_t N = b.natoms;
@@ -258,17 +309,24 @@ static nbl_status layout_workspace(Plan &p, const Batch &b) {
     size_t o_table = L.add(sizeof(int2) * b.table_size);
     size_t o_hkey = b.grid == kGridHashed ? L.add(sizeof(unsigned long long) * b.table_size) : 0;
     size_t o_pos64 = L.add(sizeof(double4) * N);
-    size_t o_pos32 = L.add(sizeof(float4) * N);
+    size_t o_pos32 = L.add(sizeof(float4) * (N + 32));  // read in whole groups of eight
     size_t o_aux = L.add(sizeof(int4) * N);
     size_t o_amax = L.add(sizeof(float) * nsys);
     size_t o_home = L.add(sizeof(HomeCell) * N);
     size_t o_cnt = L.add(sizeof(int32_t) * (N + 1));
     // row offsets, then the 8-int flag block right after offsets[N]
     size_t o_off = L.add(sizeof(int64_t) * (N + 1) + sizeof(int) * 8);
-    const int64_t mask_cap = mask_words(p, b);
+    // the row passes' lists, or the warp passes' hit words and work items
+    const int64_t mask_cap = p.rows ? 0 : mask_words(p, b);
     size_t o_mask = L.add(sizeof(uint32_t) * mask_cap);
-    size_t o_hmask = L.add(sizeof(long long) * std::max<int64_t>(N, 1) * kMaskBatches);
-    size_t o_items = L.add(sizeof(WorkItem) * std::max<int64_t>(N, 1));
+    size_t o_hmask =
+        p.rows ? 0 : L.add(sizeof(long long) * std::max<int64_t>(N, 1) * kMaskBatches);
+    size_t o_items = p.sparse ? 0 : L.add(sizeof(WorkItem) * std::max<int64_t>(N, 1));
+    const ListPlan lp = p.rows ? plan_lists(p, b) : ListPlan();
+    size_t o_list = L.add(sizeof(uint4) * lp.total);
+    size_t o_hcell = p.rows ? L.add(sizeof(int4) * N) : 0;
+    size_t o_inv = p.rows ? L.add(sizeof(int32_t) * N) : 0;
+    size_t o_rowof = p.rows ? L.add(sizeof(int32_t) * lp.row_cap) : 0;
     size_t o_ljp = L.add(sizeof(double) * (size_t)(std::max<int64_t>(N, 1) + N / 1024 + 64));
     nbl_status st = ensure(p.ws.base, p.ws.bytes, L.total, "workspace");
     if (st != NBL_SUCCESS) {
@@ -312,10 +370,15 @@ static nbl_status layout_workspace(Plan &p, const Batch &b) {
     B.counts = (int32_t *)at(o_cnt);
     B.offsets = (int64_t *)at(o_off);
     B.small = reinterpret_cast<int *>(B.offsets + N + 1);
-    B.mask_pool = (uint32_t *)at(o_mask);
+    B.mask_pool = p.rows ? nullptr : (uint32_t *)at(o_mask);
     B.mask_cap = mask_cap;
-    B.home_mask = (long long *)at(o_hmask);
-    B.items = (WorkItem *)at(o_items);
+    B.home_mask = p.rows ? nullptr : (long long *)at(o_hmask);
+    B.items = p.sparse ? nullptr : (WorkItem *)at(o_items);
+    B.list = p.rows ? (uint4 *)at(o_list) : nullptr;
+    B.hcell = p.rows ? (int4 *)at(o_hcell) : nullptr;
+    B.inv = p.rows ? (int32_t *)at(o_inv) : nullptr;
+    B.row_of = p.rows ? (int32_t *)at(o_rowof) : nullptr;
+    B.list_plan = lp;
     B.lj_part = (double *)at(o_ljp);
     return NBL_SUCCESS;
 }
@@ -385,10 +448,10 @@ nbl_status finish_batch(Batch &b, int grid_req) {
 // items in a fixed stride, so a grid that is not a whole number of waves
 // leaves its last partial wave running alone.
 static int traverse_grid(const Plan &p, int64_t natoms, int mult, int mode, bool fp32,
-                         int kind, const TravShape &shape, bool lj) {
+                         int kind, const TravShape &shape) {
     if (mult <= 0)
-        mult = kAutoWaves * std::max(1, traverse_blocks_per_sm(mode, fp32, kind, shape, lj,
-                                                               p.targs.runs != 0));
+        mult = kAutoWaves *
+               std::max(1, traverse_blocks_per_sm(mode, fp32, kind, shape, p.targs.runs != 0));
     const int64_t items = std::max<int64_t>((natoms + 3) / 4, 1);
     return (int)std::min<int64_t>((int64_t)p.num_sms * mult, items);
 }
@@ -398,13 +461,27 @@ static int traverse_grid(const Plan &p, int64_t natoms, int mult, int mode, bool
 // plain FP64 sweep reads each segment's own offset) and the systems' visit
 // tables (a pair's offset vector is looked up there).
 static int run_limit(const Plan &p, const Batch &b) {
-    if (b.grid != kGridDense || !b.fp32 || p.bufs.visit == nullptr) return 1;
+    if (p.rows || b.grid != kGridDense || !b.fp32 || p.bufs.visit == nullptr) return 1;
     // left to the device only where the grid is sparse on average (below two
     // atoms per cell); denser grids keep one cell per item and the kernels
     // without run handling
     if (p.max_run == 0 && (double)b.natoms >= 2.0 * (double)b.table_size) return 1;
     return p.max_run;
 }
+
+// Atoms of the cells that an atom of batch b visits, on average.
+static double candidates_per_atom(const Batch &b) {
+    double cand = 0.0;
+    for (size_t s = 0; s < b.sys.size(); s++)
+        cand += (double)b.sys[s].nat * b.sys[s].nvisit * b.sys[s].nat /
+                (double)std::max<int64_t>(b.ncells[s], 1);
+    return cand / (double)std::max<int64_t>(b.natoms, 1);
+}
+
+// Candidates per atom above which the list count drops those outside the
+// tile's bounding box before staging: two full tables.  Measured with and
+// without: 1,548 / 2,411 us at about 3,000, 527 / 490 us at 300.
+constexpr double kCullCand = 832.0;
 
 // Atoms per work item (the cell-occupancy tile) for batch b: the launch
 // configuration's, or by default chosen from the atom count.  A small system
@@ -431,9 +508,9 @@ static int tile_of(const Plan &p, const Batch &b) {
 // cells stands in for it.  Measured on 200,000-atom uniform gases (count +
 // fill): 2.7x faster at 0.25 atoms per cell (1.1 per occupied cell), 2.0x at
 // 0.5 (1.3), 1.35x at 1 (1.6), even at 2 (2.3), slower above; even on a slab
-// of 2 atoms per occupied cell.  The force sink always takes the work items.
+// of 2 atoms per occupied cell.  The force pass has its own rule (lj_atom_mode).
 static bool atom_mode(const Plan &p, const Batch &b) {
-    if (p.no_atoms || p.atom_threads < 0 || p.bufs.visit == nullptr) return false;
+    if (p.atom_threads < 0 || p.bufs.visit == nullptr) return false;
     if (p.atom_threads > 0) return true;
     if (p.occ_cells > 0 && p.occ_natoms == b.natoms && p.occ_table == b.table_size)
         return (double)b.natoms < 2.0 * (double)p.occ_cells;
@@ -442,8 +519,33 @@ static bool atom_mode(const Plan &p, const Batch &b) {
     return (double)b.natoms < cells;
 }
 
+// Whether the count takes one thread per atom (nbl_rows.cu) instead of one warp
+// per cell: where the occupied cells hold few atoms.
+static bool sparse_grid(const Plan &p, const Batch &b) {
+    if (p.occ_cells > 0 && p.occ_natoms == b.natoms && p.occ_table == b.table_size)
+        return (double)b.natoms < kSparseAtoms * (double)p.occ_cells;
+    double cells = 0.0;
+    for (int64_t n : b.ncells) cells += (double)n;
+    return (double)b.natoms < kSparseAtoms * cells;
+}
+
+// Whether the Lennard-Jones pass runs one thread per atom: it needs no second
+// walk to write pairs, so the line lies higher than the list's.
+static bool lj_atom_mode(const Plan &p, const Batch &b) {
+    if (p.atom_threads < 0 || p.bufs.visit == nullptr) return false;
+    if (p.atom_threads > 0) return true;
+    double cells = 0.0;
+    for (int64_t n : b.ncells) cells += (double)n;
+    return (double)b.natoms < kLjAtomsPerCell * cells;
+}
+
 // Size the workspace for a batch and copy its inputs and host tables in.
-nbl_status upload_batch(Plan &p, const Batch &b, cudaStream_t st) {
+nbl_status upload_batch(Plan &p, const Batch &b, cudaStream_t st, bool one_launch) {
+    // the row passes, unless the one-launch count phase or the launch
+    // configuration asks for the warp passes or the thread-per-atom passes
+    p.rows = !one_launch && p.atom_threads == 0 && p.max_run == 0;
+    p.sparse = p.rows && (!b.fp32 || sparse_grid(p, b));
+    p.cand_atom = candidates_per_atom(b);
     nbl_status s = layout_workspace(p, b);
     if (s != NBL_SUCCESS) return s;
     Bufs &B = p.bufs;
@@ -454,6 +556,8 @@ nbl_status upload_batch(Plan &p, const Batch &b, cudaStream_t st) {
     p.batch_fp32 = b.fp32;
     p.batch_grid = b.grid;
     p.have_count = false;
+    p.count_pending = false;
+    p.lists_short = true;  // until a synchronised count says otherwise
 
     if (!b.pos_on_device && N > 0)
         NBL_CUDA(cudaMemcpyAsync(B.pos, b.positions, sizeof(double) * 3 * N,
@@ -484,6 +588,16 @@ nbl_status upload_batch(Plan &p, const Batch &b, cudaStream_t st) {
         // the same layout as the device block at B.sys: one copy
         char *h = static_cast<char *>(p.host_stage);
         std::memcpy(h, b.sys.data(), sizeof(SysDev) * nsys);
+        if (p.rows) {
+            SysDev *hs = reinterpret_cast<SysDev *>(h);
+            int64_t at = 0;
+            for (int s2 = 0; s2 < nsys; s2++) {
+                const int64_t cap = B.list_plan.cap(expected_row(b, s2));
+                hs[s2].list_base = at;
+                hs[s2].list_cap = (int32_t)cap;
+                at += cap * hs[s2].nat;
+            }
+        }
         if (B.visit != nullptr) {
             SysDev *hs = reinterpret_cast<SysDev *>(h);
             int64_t base = 0;
@@ -543,12 +657,16 @@ static void gather_args(const Plan &p, const Batch &b, const uint32_t *skeys,
     ga.pos64 = B.pos64;
     ga.pos32 = B.pos32;
     ga.aux = B.aux;
+    ga.hcell = B.hcell;
+    ga.unroll = p.sparse ? 1 : 0;
+    ga.err = B.small + 1;
+    ga.inv = B.inv;
     ga.amax = B.amax;
     ga.home = B.home;
     ga.n_home = B.small + 0;
 }
 
-static void traverse_args(Plan &p, const Batch &b) {
+static void traverse_args(Plan &p, const Batch &b, bool atoms, int max_run) {
     const Bufs &B = p.bufs;
     const int64_t N = b.natoms;
     TraverseArgs &ta = p.targs;
@@ -582,22 +700,32 @@ static void traverse_args(Plan &p, const Batch &b) {
     ta.i_hi = p.i_hi;
     ta.itile = tile_of(p, b);
     ta.natoms = N;
-    ta.runs = run_limit(p, b) != 1 ? 1 : 0;
-    ta.atoms = atom_mode(p, b) ? 1 : 0;
+    ta.runs = max_run != 1 ? 1 : 0;
+    ta.atoms = atoms ? 1 : 0;
     ta.sys_atom_base = B.sys_atom_base;
     ta.nsys = (int)b.sys.size();
+    ta.list = B.list;
+    ta.list_chunks = B.list_plan.chunks;
+    ta.list_cap = B.list_plan.total;
+    ta.list_wide = B.list_plan.wide ? 1 : 0;
+    ta.list_shift = B.list_plan.shift;
+    ta.hcell = B.hcell;
+    ta.inv = B.inv;
+    ta.row_of = B.row_of;
+    ta.row_cap = B.list_plan.row_cap;
     p.batch_kind = b.sys.empty() ? kCutScalar : b.sys[0].cutoff_kind;
     p.trav_grid = traverse_grid(p, N, p.count_mult, kModeCount, b.fp32, p.batch_kind,
-                                p.count_shape, false);
+                                p.count_shape);
     p.fill_grid = traverse_grid(p, N, p.fill_mult, kModeFill, b.fp32, p.batch_kind,
-                                p.fill_shape, false);
+                                p.fill_shape);
 }
 
-// Enqueue the count phase (bin, sort, gather, work items, count, scan) on a
-// batch whose inputs are resident: no host synchronisation, no allocation,
-// so it can be captured in a CUDA graph.
-nbl_status enqueue_count(Plan &p, const Batch &b, cudaStream_t st) {
-    StageRange whole("nbl.count_phase");
+// Enqueue the stages before the pair passes (bin, sort, gather, work items)
+// on a batch whose inputs are resident: no host synchronisation, no
+// allocation, so it can be captured in a CUDA graph.  atoms: the passes will
+// run one thread per atom (no work items); max_run: cells per work item.
+static nbl_status enqueue_build(Plan &p, const Batch &b, bool atoms, int max_run,
+                                cudaStream_t st) {
     Bufs &B = p.bufs;
     const int64_t N = b.natoms;
     const int nsys = (int)b.sys.size();
@@ -619,32 +747,77 @@ nbl_status enqueue_count(Plan &p, const Batch &b, cudaStream_t st) {
     }
     GatherArgs ga;
     gather_args(p, b, in_alt ? B.keys2 : B.keys, in_alt ? B.vals2 : B.vals, ga);
-    const bool atoms = atom_mode(p, b);
     {
         StageRange r("nbl.gather");
         NBL_CUDA(launch_gather(ga, st), "k_gather");
-        if (!atoms)  // the thread-per-atom passes need no work items
+        if (!atoms && !p.sparse)  // passes by atoms and sparse counts need no work items
             NBL_CUDA(launch_tiles(B.home, ga.n_home, B.table, B.sys, B.items, B.small + 3, N,
-                                  p.num_sms, tile_of(p, b), run_limit(p, b), st),
+                                  p.num_sms, tile_of(p, b), max_run, st),
                      "k_tiles");
     }
-    traverse_args(p, b);
+    traverse_args(p, b, atoms, max_run);
     p.targs.skeys = in_alt ? B.keys2 : B.keys;
+    return NBL_SUCCESS;
+}
+
+// The count pass and the row offsets over the stages enqueue_build left
+// (ticket_ready: the work-item ticket is still clear).
+static nbl_status enqueue_count_pass(Plan &p, bool ticket_ready, cudaStream_t st) {
+    Bufs &B = p.bufs;
+    const int64_t N = p.batch_natoms;
     if (p.i_lo > 0 || p.i_hi < N)
         NBL_CUDA(cudaMemsetAsync(B.counts, 0, sizeof(int32_t) * N, st), "memset counts");
     {
         StageRange r("nbl.count");
         TraverseArgs tc = p.targs;
-        tc.ticket_ready = 1;  // k_init cleared the ticket
-        NBL_CUDA(launch_traverse(kModeCount, b.fp32, p.batch_kind, tc, p.trav_grid, st,
+        tc.ticket_ready = ticket_ready ? 1 : 0;
+        if (p.sparse)
+            NBL_CUDA(launch_count_rows(p.batch_fp32, p.batch_kind, tc, st), "count pass");
+        else if (p.rows)
+            NBL_CUDA(launch_count_list(p.batch_kind, p.cand_atom > kCullCand, tc, p.num_sms, st),
+                     "count pass");
+        else
+        NBL_CUDA(launch_traverse(kModeCount, p.batch_fp32, p.batch_kind, tc, p.trav_grid, st,
                                  p.count_shape),
                  "count pass");
     }
     {
         StageRange r("nbl.scan");
         NBL_CUDA(exclusive_scan_i32_i64(B.counts, N, B.offsets, B.scan64, st), "scan");
+        if (p.rows) NBL_CUDA(launch_row_marks(p.targs, st), "row marks");
     }
     return NBL_SUCCESS;
+}
+
+// Enqueue the whole count phase (bin, sort, gather, work items, count, scan).
+nbl_status enqueue_count(Plan &p, const Batch &b, cudaStream_t st) {
+    StageRange whole("nbl.count_phase");
+    const nbl_status s =
+        enqueue_build(p, b, !p.rows && atom_mode(p, b), run_limit(p, b), st);
+    return s == NBL_SUCCESS ? enqueue_count_pass(p, true, st) : s;  // k_init cleared the ticket
+}
+
+// After a force pass the plan holds the sorted atoms but no counts yet: the
+// calls that read them have them made here.
+static nbl_status ensure_counts(Plan &p, cudaStream_t st) {
+    if (!p.count_pending) return NBL_SUCCESS;
+    p.count_pending = false;
+    return enqueue_count_pass(p, false, st);
+}
+
+// What a synchronised count found: its hit-word or list demand, and how its
+// pairs compare with the density's estimate.
+void note_lists(Plan &p, const Batch &b, int64_t npairs, int64_t demand, int flags) {
+    p.lists_short = (flags & kErrNoList) != 0;
+    if (!p.rows) {
+        p.mask_hint = demand;
+        return;
+    }
+    p.list_natoms = b.natoms;
+    p.list_table = b.table_size;
+    p.list_hint = demand;
+    const double e = p.bufs.list_plan.expect;
+    p.list_scale = e > 0.0 ? std::min((double)npairs / e, 1e3) : 1.0;
 }
 
 // Whether batch b takes the one-launch count phase (nbl_small.cu): one system of
@@ -665,8 +838,7 @@ static nbl_status enqueue_count_small(Plan &p, const Batch &b, cudaStream_t st) 
     SmallCountArgs sa;
     bin_args(p, b, sa.bin);
     gather_args(p, b, B.keys, B.vals, sa.gather);
-    traverse_args(p, b);
-    p.targs.atoms = 0;  // the one-launch count builds work items for the warp passes
+    traverse_args(p, b, false, run_limit(p, b));
     // Work items of at most 8 atoms: a small system's passes are bound by the
     // latency of one item, which shrinks with its tile (100 atoms: 74 -> 62 us
     // for count + fill + synchronisation against 32-atom items).
@@ -698,7 +870,10 @@ static CountKey count_key(const Plan &p, const Batch &b) {
     k.types = p.bufs.types;
     k.natoms = b.natoms;
     k.table_size = b.table_size;
-    k.mask_cap = p.bufs.mask_cap;
+    k.mask_cap = p.rows ? p.bufs.list_plan.total : p.bufs.mask_cap;
+    k.list_chunks = p.rows ? p.bufs.list_plan.chunks : -1;
+    k.sparse = (p.sparse ? 1 : 0) | (p.bufs.list_plan.wide ? 2 : 0) |
+               p.bufs.list_plan.shift << 2;
     k.pt_size = (int64_t)b.pt64.size();
     k.i_lo = p.i_lo;
     k.i_hi = p.i_hi;
@@ -715,7 +890,7 @@ static CountKey count_key(const Plan &p, const Batch &b) {
     k.count_cand = p.count_shape.cand;
     k.count_group = p.count_shape.group;
     k.count_tickets = p.count_tickets ? 1 : 0;
-    k.atoms = atom_mode(p, b) ? 1 : 0;
+    k.atoms = !p.rows && atom_mode(p, b) ? 1 : 0;
     return k;
 }
 
@@ -760,9 +935,9 @@ static bool capture_count(Plan &p, const Batch &b, const CountKey &k) {
 }
 
 nbl_status run_count(Plan &p, const Batch &b, cudaStream_t st, bool sync) {
-    nbl_status s = upload_batch(p, b, st);
-    if (s != NBL_SUCCESS) return s;
     const bool small = sync && small_path(p, b);
+    nbl_status s = upload_batch(p, b, st, small);
+    if (s != NBL_SUCCESS) return s;
     // Single calls: replay the captured count phase while the launch key
     // repeats (captured on the second call with the same key); a small
     // system's count phase is one launch already.
@@ -787,7 +962,7 @@ nbl_status run_count(Plan &p, const Batch &b, cudaStream_t st, bool sync) {
         p.batch_kind = p.graph_kind;
         // the fill's shape is not part of the count key
         p.fill_grid = traverse_grid(p, b.natoms, p.fill_mult, kModeFill, b.fp32, p.batch_kind,
-                                    p.fill_shape, false);
+                                    p.fill_shape);
         NBL_CUDA(cudaGraphLaunch(p.count_graph, st), "count-phase graph");
         count_launch((int)p.graph_launches);
     } else {
@@ -812,7 +987,7 @@ nbl_status run_count(Plan &p, const Batch &b, cudaStream_t st, bool sync) {
         }
         unsigned long long demand = 0;  // mask-pool words the count asked for
         std::memcpy(&demand, flags + 4, sizeof(demand));
-        p.mask_hint = (int64_t)demand;
+        note_lists(p, b, p.npairs, (int64_t)demand, flags[1]);
         if (flags[1] & kErrRange)
             return set_error(NBL_ERROR_RANGE,
                              "positions must be finite and within 2^29 cells of the box");
@@ -826,6 +1001,8 @@ nbl_status run_count(Plan &p, const Batch &b, cudaStream_t st, bool sync) {
 nbl_status run_fill(Plan &p, const nbl_outputs &o, int64_t capacity, cudaStream_t st) {
     if (!p.have_count)
         return set_error(NBL_ERROR_INVALID_ARGUMENT, "nbl_fill without a preceding nbl_count");
+    const nbl_status counted = ensure_counts(p, st);
+    if (counted != NBL_SUCCESS) return counted;
     TraverseArgs ta = p.targs;
     ta.item_next = p.fill_tickets ? p.bufs.small + 6 : nullptr;
     ta.first = o.first;
@@ -836,6 +1013,12 @@ nbl_status run_fill(Plan &p, const nbl_outputs &o, int64_t capacity, cudaStream_
     ta.capacity = capacity;
     if (!(o.first || o.second || o.distvec || o.absdist || o.shift)) return NBL_SUCCESS;
     StageRange r("nbl.fill");
+    if (p.rows) {
+        NBL_CUDA(launch_fill_rows(ta, p.num_sms, st), "fill pass");
+        // rows without a list (none where a synchronised count said so)
+        if (p.lists_short) NBL_CUDA(launch_fill_atoms(p.batch_kind, ta, st), "fill pass");
+        return NBL_SUCCESS;
+    }
     NBL_CUDA(launch_traverse(kModeFill, p.batch_fp32, p.batch_kind, ta, p.fill_grid, st,
                              p.fill_shape),
              "fill pass");
@@ -1222,13 +1405,17 @@ nbl_status nbl_fill_matrix(nbl_plan *plan, int32_t max_neighbours, int32_t *idx,
     if (!p.have_count) return set_error(NBL_ERROR_INVALID_ARGUMENT, "no count phase");
     DeviceGuard g(p.device);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const nbl_status counted = ensure_counts(p, st);
+    if (counted != NBL_SUCCESS) return counted;
     const int64_t n = p.batch_natoms;
     const size_t nk = (size_t)n * (size_t)max_neighbours;
     *overflow = 0;
     if (n == 0) return NBL_SUCCESS;
-    NBL_CUDA(cudaMemsetAsync(idx, 0, sizeof(int32_t) * nk, st), "memset matrix");
-    NBL_CUDA(cudaMemsetAsync(dist, 0, sizeof(double) * 3 * nk, st), "memset matrix");
-    NBL_CUDA(cudaMemsetAsync(count, 0, sizeof(int32_t) * n, st), "memset matrix");
+    if (!p.rows) {  // the row pass writes every slot itself
+        NBL_CUDA(cudaMemsetAsync(idx, 0, sizeof(int32_t) * nk, st), "memset matrix");
+        NBL_CUDA(cudaMemsetAsync(dist, 0, sizeof(double) * 3 * nk, st), "memset matrix");
+        NBL_CUDA(cudaMemsetAsync(count, 0, sizeof(int32_t) * n, st), "memset matrix");
+    }
     NBL_CUDA(cudaMemsetAsync(p.bufs.small + 2, 0, sizeof(int), st), "memset flag");
     TraverseArgs ta = p.targs;
     ta.item_next = p.fill_tickets ? p.bufs.small + 6 : nullptr;
@@ -1238,9 +1425,14 @@ nbl_status nbl_fill_matrix(nbl_plan *plan, int32_t max_neighbours, int32_t *idx,
     ta.mat_count = count;
     ta.mat_overflow = p.bufs.small + 2;
     ta.capacity = 0;
-    NBL_CUDA(launch_traverse(kModeFill, p.batch_fp32, p.batch_kind, ta, p.fill_grid, st,
-                             p.fill_shape),
-             "matrix fill");
+    if (p.rows) {
+        NBL_CUDA(launch_fill_rows(ta, p.num_sms, st), "matrix fill");
+        if (p.lists_short) NBL_CUDA(launch_fill_atoms(p.batch_kind, ta, st), "matrix fill");
+    } else {
+        NBL_CUDA(launch_traverse(kModeFill, p.batch_fp32, p.batch_kind, ta, p.fill_grid, st,
+                                 p.fill_shape),
+                 "matrix fill");
+    }
     NBL_CUDA(cudaMemcpyAsync(p.host_small + 2, p.bufs.small + 2, sizeof(int),
                              cudaMemcpyDeviceToHost, st), "read overflow");
     nbl_status r = read_flags(p, st);
@@ -1268,28 +1460,27 @@ nbl_status nbl_lj_forces(nbl_plan *plan, const nbl_request *req, double epsilon,
     if (!g.ok) return set_error(NBL_ERROR_CUDA, "cannot select device %d", plan->p.device);
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
     Plan &p = plan->p;
-    p.no_atoms = true;  // the force sink takes the work items
-    st = run_count(p, b, cs, false);
-    p.no_atoms = false;
+    st = upload_batch(p, b, cs, false);
     if (st != NBL_SUCCESS) return st;
+    const bool atoms = lj_atom_mode(p, b);
+    st = enqueue_build(p, b, atoms, 1, cs);
+    if (st != NBL_SUCCESS) return st;
+    p.have_count = true;
+    p.count_pending = true;
     if (b.natoms == 0) {
         NBL_CUDA(cudaMemsetAsync(energy, 0, sizeof(double), cs), "memset energy");
         return NBL_SUCCESS;
     }
     TraverseArgs ta = p.targs;
     ta.item_next = p.fill_tickets ? p.bufs.small + 6 : nullptr;
-    ta.first = ta.second = nullptr;
-    ta.distvec = ta.absdist = nullptr;
-    ta.shift = nullptr;
-    ta.capacity = 0;
+    ta.ticket_ready = 1;  // k_init cleared the ticket
     ta.lj_force = forces;
     ta.lj_energy = p.bufs.lj_part;
     ta.lj_eps4 = 4.0 * epsilon;
     ta.lj_eps24 = 24.0 * epsilon;
     ta.lj_sig2 = sigma * sigma;
-    const int grid = traverse_grid(p, b.natoms, p.fill_mult, kModeFill, p.batch_fp32,
-                                   p.batch_kind, TravShape(), true);
-    NBL_CUDA(launch_traverse(kModeFill, p.batch_fp32, p.batch_kind, ta, grid, cs),
+    NBL_CUDA(atoms ? launch_lj_atoms(p.batch_kind, ta, cs)
+                   : launch_lj_items(p.batch_kind, ta, p.num_sms, cs),
              "force pass");
     NBL_CUDA(launch_lj_energy(p.bufs.lj_part, b.natoms, p.bufs.lj_part + b.natoms, energy,
                               cs),
@@ -1303,6 +1494,8 @@ nbl_status nbl_counts(nbl_plan *plan, int32_t *counts, void *stream) {
     Plan &p = plan->p;
     if (!p.have_count) return set_error(NBL_ERROR_INVALID_ARGUMENT, "no count phase");
     DeviceGuard g(p.device);
+    const nbl_status counted = ensure_counts(p, static_cast<cudaStream_t>(stream));
+    if (counted != NBL_SUCCESS) return counted;
     if (p.batch_natoms > 0)
         NBL_CUDA(cudaMemcpyAsync(counts, p.bufs.counts, sizeof(int32_t) * p.batch_natoms,
                                  cudaMemcpyDeviceToDevice, static_cast<cudaStream_t>(stream)),
@@ -1316,6 +1509,8 @@ nbl_status nbl_row_offsets(nbl_plan *plan, int64_t *offsets, void *stream) {
     Plan &p = plan->p;
     if (!p.have_count) return set_error(NBL_ERROR_INVALID_ARGUMENT, "no count phase");
     DeviceGuard g(p.device);
+    const nbl_status counted = ensure_counts(p, static_cast<cudaStream_t>(stream));
+    if (counted != NBL_SUCCESS) return counted;
     NBL_CUDA(cudaMemcpyAsync(offsets, p.bufs.offsets, sizeof(int64_t) * (p.batch_natoms + 1),
                              cudaMemcpyDeviceToDevice, static_cast<cudaStream_t>(stream)),
              "copy offsets");

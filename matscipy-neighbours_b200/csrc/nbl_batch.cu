@@ -374,6 +374,26 @@ bool tune_for_tile(nbl_batch *bt, cudaStream_t st, cudaEvent_t e0, cudaEvent_t e
     return true;
 }
 
+// The row passes have one launch shape; the tile size is the count's only
+// choice.  (The other fields report the default shapes at two waves.)
+bool tune_rows(nbl_batch *bt, cudaStream_t st, cudaEvent_t e0, cudaEvent_t e1, int itile,
+               TuneChoice &best) {
+    Plan &p = bt->p;
+    const int kind = bt->b.sys.empty() ? kCutScalar : bt->b.sys[0].cutoff_kind;
+    TuneChoice c;
+    c.itile = itile;
+    c.count_mult = 2 * std::max(1, traverse_blocks_per_sm(kModeCount, bt->b.fp32, kind, TravShape()));
+    c.fill_mult = 2 * std::max(1, traverse_blocks_per_sm(kModeFill, bt->b.fp32, kind, TravShape()));
+    apply_choice(p, c);
+    c.count_ms = time_count(bt, st, e0, e1);
+    if (c.count_ms >= 1e30f) return false;
+    p.have_count = true;  // the fills below read this count's offsets
+    c.fill_ms = time_fill(bt, st, e0, e1);
+    if (c.fill_ms >= 1e30f) return false;
+    best = c;
+    return true;
+}
+
 nbl_status autotune(nbl_batch *bt, cudaStream_t st) {
     const Batch &b = bt->b;
     double cells = 0.0;
@@ -383,7 +403,8 @@ nbl_status autotune(nbl_batch *bt, cudaStream_t st) {
         max_visit = std::max(max_visit, b.sys[s].nvisit);
     }
     char key[160];
-    std::snprintf(key, sizeof(key), "w5_sm%d_k%d_f%d_d%d_v%d", bt->p.num_sms,
+    std::snprintf(key, sizeof(key), "%s_sm%d_k%d_f%d_d%d_v%d",
+                  bt->p.rows ? "r1" : "w5", bt->p.num_sms,
                   b.sys.empty() ? 0 : b.sys[0].cutoff_kind, b.fp32 ? 1 : 0,
                   bucket_log2(b.natoms / std::max(cells, 1.0)), bucket_log2(max_visit));
     bt->tune_key = key;
@@ -406,7 +427,9 @@ nbl_status autotune(nbl_batch *bt, cudaStream_t st) {
     const int tiles[] = {32, 16};
     for (int t : tiles) {
         TuneChoice c;
-        if (!tune_for_tile(bt, st, e0, e1, t, c)) continue;
+        if (!(bt->p.rows ? tune_rows(bt, st, e0, e1, t, c)
+                         : tune_for_tile(bt, st, e0, e1, t, c)))
+            continue;
         if (!have || c.count_ms + c.fill_ms < best.count_ms + best.fill_ms) best = c;
         have = true;
     }
@@ -521,8 +544,8 @@ NBL_API nbl_status nbl_batch_setup(nbl_batch *bt, const nbl_batch_request *req,
         std::memcpy(flags, bt->p.host_small + 1, sizeof(flags));
         unsigned long long demand = 0;
         std::memcpy(&demand, flags + 4, sizeof(demand));
-        if ((long long)demand > bt->p.bufs.mask_cap) {
-            bt->p.mask_hint = (int64_t)demand;
+        note_lists(bt->p, b, bt->p.host_small[0], (int64_t)demand, flags[1]);
+        if (bt->p.rows || (long long)demand > bt->p.bufs.mask_cap) {
             s = upload_batch(bt->p, b, st);
             if (s != NBL_SUCCESS) return s;
             NBL_CUDA(cudaStreamSynchronize(st), "batch upload");

@@ -193,25 +193,24 @@ bool traverse_shape_ok(int mode, bool fp32, const TravShape &s) {
     return (s.cand == 0 || s.cand == 1) && (!fp32 || s.group == 2 || s.group == 4);
 }
 
-int traverse_blocks_per_sm(int mode, bool fp32, int kind, const TravShape &shape, bool lj,
-                           bool runs) {
+int traverse_blocks_per_sm(int mode, bool fp32, int kind, const TravShape &shape, bool runs) {
     // cached per device, pass, precision, kind, shape and run instantiation
     constexpr int kDev = 16;
-    static std::atomic<int> cache[kDev][2][2][3][3][2][2][2][2];
+    static std::atomic<int> cache[kDev][2][2][3][3][2][2][2];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDev) {
         cudaGetLastError();
         dev = -1;
     }
     const int mi = mode == kModeCount ? 0 : 1, fi = fp32 ? 1 : 0;
-    const int ki = kind == kCutPerAtom ? 1 : (kind == kCutPerType ? 2 : 0), li = lj ? 1 : 0;
+    const int ki = kind == kCutPerAtom ? 1 : (kind == kCutPerType ? 2 : 0);
     const int wi = shape.warps == 2 ? 0 : (shape.warps == 8 ? 2 : 1);
     const int ci = shape.cand != 0 ? 1 : 0;
     const int gi = shape.group == 2 ? 0 : 1;
     runs = runs && fp32;  // runs are only built for the FP32 filter
     const int ri = runs ? 1 : 0;
     if (dev >= 0) {
-        const int c = cache[dev][mi][fi][ki][wi][ci][gi][li][ri].load(std::memory_order_relaxed);
+        const int c = cache[dev][mi][fi][ki][wi][ci][gi][ri].load(std::memory_order_relaxed);
         if (c > 0) return c;
     }
     int n = 0;
@@ -220,11 +219,11 @@ int traverse_blocks_per_sm(int mode, bool fp32, int kind, const TravShape &shape
                   : (runs ? occupancy_count_fp32_runs(kind, shape)
                           : occupancy_count_fp32(kind, shape));
     else
-        n = !fp32 ? occupancy_fill_fp64(kind, shape, lj)
-                  : (runs ? occupancy_fill_fp32_runs(kind, shape, lj)
-                          : occupancy_fill_fp32(kind, shape, lj));
+        n = !fp32 ? occupancy_fill_fp64(kind, shape)
+                  : (runs ? occupancy_fill_fp32_runs(kind, shape)
+                          : occupancy_fill_fp32(kind, shape));
     if (dev >= 0 && n > 0)
-        cache[dev][mi][fi][ki][wi][ci][gi][li][ri].store(n, std::memory_order_relaxed);
+        cache[dev][mi][fi][ki][wi][ci][gi][ri].store(n, std::memory_order_relaxed);
     return n;
 }
 
@@ -233,7 +232,6 @@ cudaError_t launch_traverse(int mode, bool fp32, int kind, const TraverseArgs &a
     if (grid <= 0) return cudaSuccess;
     if (!traverse_shape_ok(mode, fp32, shape)) return cudaErrorInvalidValue;
     if (a.atoms) {  // one thread per atom; precision does not apply (exact FP64)
-        if (a.lj_force != nullptr) return cudaErrorInvalidValue;
         return mode == kModeCount ? launch_count_atoms(kind, a, st)
                                   : launch_fill_atoms(kind, a, st);
     }

@@ -41,6 +41,10 @@ struct GatherArgs {
     double4 *pos64;
     float4 *pos32;
     int4 *aux;
+    int4 *hcell;              // [natoms] home cell and system per sorted atom, or null
+    int32_t *inv;             // [natoms] sorted index of each atom, or null
+    int unroll;               // pos32 unrolled along x (the row passes' frame)
+    int *err;
     float *amax;              // [nsys], zeroed
     HomeCell *home;
     int *n_home;              // zeroed
@@ -90,10 +94,9 @@ struct TraverseArgs {
     double *mat_dist;
     int32_t *mat_count;
     int *mat_overflow;
-    // Force sink (lj_force != nullptr): instead of writing pairs, the fill
-    // pass sums Lennard-Jones forces per atom i into lj_force[3 * atom] and
-    // its energy share (1/2 U per pair of its row) into lj_energy[atom];
-    // every in-range atom is written once.
+    // Force passes (launch_lj_*): Lennard-Jones forces per atom i into
+    // lj_force[3 * atom] and its energy share (1/2 U per pair of its row) into
+    // lj_energy[atom]; every in-range atom is written once.
     double *lj_force;
     double *lj_energy;
     double lj_eps4, lj_eps24, lj_sig2;
@@ -123,7 +126,22 @@ struct TraverseArgs {
     const uint32_t *skeys;          // sorted cell keys (the sort's output)
     const int64_t *sys_atom_base;   // first atom of each system
     int nsys;
+    // Neighbour lists of the row passes (nbl_rows.cu): 16-byte groups of one- or
+    // (list_wide) two-word entries, of which those from list_chunks on are
+    // handed out in chunks (mask_cursor); the sorted
+    // atoms' home cells and systems, the sorted index of each atom, and the
+    // row of every kRowChunk-th output slot.
+    uint4 *list;
+    long long list_chunks, list_cap;
+    int list_wide, list_shift;
+    const int4 *hcell;
+    const int32_t *inv;
+    int32_t *row_of;
+    long long row_cap;
 };
+
+constexpr int kListChunk = 16;   // groups per chained chunk, the link included
+constexpr int kRowChunk = 256;   // output slots a fill warp takes at a time
 
 // Launch shape of one pair pass: warps per CTA (2, 4 or 8, i.e. 64, 128 or
 // 256 threads), candidates staged per warp in the count (cand 0: 384 FP32 /
@@ -194,11 +212,11 @@ cudaError_t launch_tiles(const HomeCell *home, const int *n_home, const int2 *ta
                          int num_sms, int itile, int max_run, cudaStream_t st);
 cudaError_t launch_traverse(int mode, bool fp32, int kind, const TraverseArgs &a,
                             int grid, cudaStream_t st, const TravShape &shape = TravShape());
-// CTAs of the pair pass (mode, precision, cutoff kind, shape, force sink)
+// CTAs of the pair pass (mode, precision, cutoff kind, shape)
 // resident per SM on the current device: the grid of one full wave is this
 // times the SM count.  0 on error.
 int traverse_blocks_per_sm(int mode, bool fp32, int kind, const TravShape &shape = TravShape(),
-                           bool lj = false, bool runs = false);
+                           bool runs = false);
 // Candidates one count warp stages per sweep for a shape.
 constexpr int count_candidates(bool fp32, int cand) {
     return (fp32 ? 384 : 192) * (cand != 0 ? 2 : 1);
@@ -222,14 +240,25 @@ cudaError_t launch_count_fp32_runs(int kind, const TraverseArgs &a, int grid, cu
 cudaError_t launch_fill_fp32_runs(int kind, const TraverseArgs &a, int grid, cudaStream_t st,
                                   const TravShape &shape);
 int occupancy_count_fp32_runs(int kind, const TravShape &shape);
-int occupancy_fill_fp32_runs(int kind, const TravShape &shape, bool lj);
+int occupancy_fill_fp32_runs(int kind, const TravShape &shape);
 int occupancy_count_fp64(int kind, const TravShape &shape);
 // The thread-per-atom passes (TraverseArgs::atoms, nbl_trav_atoms.cu): one
 // thread per sorted atom walks its visited cells in the reference's order
-// with the exact FP64 test; the grid covers the atoms.  No force sink.
+// with the exact FP64 test; the grid covers the atoms.
 cudaError_t launch_count_atoms(int kind, const TraverseArgs &a, cudaStream_t st);
 cudaError_t launch_fill_atoms(int kind, const TraverseArgs &a, cudaStream_t st);
-int occupancy_fill_fp32(int kind, const TravShape &shape, bool lj);
-int occupancy_fill_fp64(int kind, const TravShape &shape, bool lj);
+// The row passes (nbl_rows.cu): count and lists, the row marks (after the
+// offsets are in), and the fill.
+cudaError_t launch_count_rows(bool fp32, int kind, const TraverseArgs &a, cudaStream_t st);
+cudaError_t launch_count_list(int kind, bool cull, const TraverseArgs &a, int num_sms,
+                              cudaStream_t st);
+cudaError_t launch_row_marks(const TraverseArgs &a, cudaStream_t st);
+cudaError_t launch_fill_rows(const TraverseArgs &a, int num_sms, cudaStream_t st);
+// Lennard-Jones forces (TraverseArgs::lj_*) without a count: one warp per
+// one-cell work item (nbl_lj.cu), or one thread per atom.
+cudaError_t launch_lj_items(int kind, const TraverseArgs &a, int num_sms, cudaStream_t st);
+cudaError_t launch_lj_atoms(int kind, const TraverseArgs &a, cudaStream_t st);
+int occupancy_fill_fp32(int kind, const TravShape &shape);
+int occupancy_fill_fp64(int kind, const TravShape &shape);
 
 }  // namespace nbl

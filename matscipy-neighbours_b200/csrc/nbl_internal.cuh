@@ -40,6 +40,8 @@ constexpr int kCutPerType = 2;
 constexpr int kErrRange = 1;      // non-finite or out-of-range position
 constexpr int kErrCapacity = 2;   // output slot beyond capacity
 constexpr int kErrInternal = 4;   // a device-side bound was hit
+constexpr int kErrNoList = 8;     // not an error: rows whose neighbour list did not fit
+constexpr int kNoteWideRadius = 16;  // not an error: a radius above half the binning cutoff
 
 // Checked build (-DNBL_CHECKED=1, libnbl_b200_checked.so): the traversal
 // kernels also test the indices that the release build holds in bounds by
@@ -90,6 +92,9 @@ struct SysDev {
     int32_t pt_base;     // first entry of this system's per-type tables
     int32_t nvisit;      // (2nx+1)(2ny+1)(2nz+1)
     int64_t visit_base;  // first VisitDev entry of this system, -1: computed per item
+    int64_t list_base;   // neighbour lists (nbl_rows.cu): first group of this system,
+    int32_t list_cap;    // groups per atom (the last one is the link)
+    int32_t pad_;
 };
 
 // One visited neighbour offset of a system (neighbour_visit.hh:63-84): the

@@ -258,6 +258,7 @@ extern "C" NBL_API nbl_status nbl_neighbour_list_noalloc(const nbl_request *req,
     ga.amax = amax;
     ga.home = home;
     ga.n_home = small;
+    ga.err = small + 1;
     NA_CUDA(launch_gather(ga, s), "k_gather");
     int nsm_tiles = 148;
     cudaDeviceGetAttribute(&nsm_tiles, cudaDevAttrMultiProcessorCount, dev);

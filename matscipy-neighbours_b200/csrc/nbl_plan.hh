@@ -32,6 +32,17 @@ struct Batch {
     int quantities = 0;
 };
 
+// Sizes of the row passes' neighbour lists (nbl_rows.cu).
+struct ListPlan {
+    int64_t total = 0, chunks = 0;  // 16-byte groups; first one of the chained chunks
+    bool wide = false;              // two-word entries
+    int shift = 27;                 // else: bits of the sorted atom
+    int64_t row_cap = 0;            // row marks
+    double expect = 0.0;            // pairs the density alone would give
+    double scale = 1.0, shrink = 1.0;
+    int64_t cap(double expected_row) const;  // groups per atom
+};
+
 // Device buffers of one call, carved out of the workspace.
 struct Bufs {
     double *pos = nullptr;
@@ -69,6 +80,11 @@ struct Bufs {
     long long mask_cap = 0;
     long long *home_mask = nullptr;
     WorkItem *items = nullptr;
+    uint4 *list = nullptr;         // neighbour lists, home cells, sorted indices and
+    int4 *hcell = nullptr;         // row marks of the row passes
+    int32_t *inv = nullptr;
+    int32_t *row_of = nullptr;
+    ListPlan list_plan;
     double *lj_part = nullptr;     // force sink: per-atom energies, then block sums
 };
 
@@ -83,15 +99,28 @@ struct Workspace {
 // Full waves of resident CTAs in the default grid of a pair pass.
 constexpr int kAutoWaves = 2;
 
+// Atoms above which the row of every 256th output slot is marked after the scan
+// (k_row_marks), if the pair count is known from an earlier count of the same
+// sizes (the marks' table has its size from there); below it the fill's warps search the row offsets.  Measured with and
+// without, fill + marks: 1,048,576 atoms 657 against 699 us, 200,000 27 against
+// 27, 132,651 76 against 76, 1,000 16 against 13.
+constexpr int64_t kMarkAtoms = 131072;
+// Atoms per occupied cell below which the count takes one thread per atom
+// (k_rows_count against k_count_list: 84 / 214 us at 2.3, 674 / 490 at 10).
+constexpr double kSparseAtoms = 4.0;
+
+// Atoms per cell below which the Lennard-Jones pass takes one thread per atom.
+constexpr double kLjAtomsPerCell = 1e9;
+
 // Everything that shapes the count phase's launches on a plan: when two
 // consecutive single calls have the same key, the second captures the count
 // phase into a CUDA graph and later ones replay it (compared bytewise; the
 // constructor zeroes the padding).
 struct CountKey {
     const void *ws_base, *pos, *per_atom, *types;
-    int64_t natoms, table_size, mask_cap, pt_size, i_lo, i_hi;
+    int64_t natoms, table_size, mask_cap, list_chunks, pt_size, i_lo, i_hi;
     int32_t nsys, grid, key_bits, fp32, kind, itile, max_run, nvisit_tab;
-    int32_t count_mult, count_warps, count_cand, count_group, count_tickets, atoms;
+    int32_t count_mult, count_warps, count_cand, count_group, count_tickets, atoms, sparse;
     CountKey() { std::memset(this, 0, sizeof(*this)); }
     bool operator==(const CountKey &o) const { return std::memcmp(this, &o, sizeof(*this)) == 0; }
 };
@@ -126,10 +155,8 @@ struct Plan {
     int small_atoms = kSmallDefaultAtoms;
     // Pair passes with one thread per atom (nbl_trav_atoms.cu): 0 = where the
     // occupied cells hold fewer than two atoms on average, -1 = never, 1 =
-    // always (where the systems have visit tables).  no_atoms turns them off
-    // for one count (the force sink needs the work items).
+    // always (where the systems have visit tables).
     int atom_threads = 0;
-    bool no_atoms = false;
     // Occupied cells counted by the last synchronised count, with the atom
     // count and table size it ran on (steers the default choice above).
     int64_t occ_natoms = -1, occ_table = -1, occ_cells = 0;
@@ -137,6 +164,14 @@ struct Plan {
     bool count_tickets = true;
     bool fill_tickets = true;
     int64_t mask_hint = 0;    // mask-pool words the last count asked for
+    // Row passes in use; and what the last synchronised count of these sizes
+    // found: chained entries, pairs against the density's estimate.
+    bool rows = false;
+    double cand_atom = 0.0;   // atoms of the cells that an atom visits, on average
+    bool sparse = false;      // with one thread per atom in the count
+    bool lists_short = true;  // some row may have no list (kErrNoList)
+    int64_t list_natoms = -1, list_table = -1, list_hint = 0;
+    double list_scale = 1.0;
     // Row range of nbl_set_atom_range (global atom indices, [lo, hi)).
     int64_t i_lo = 0;
     int64_t i_hi = INT64_MAX;
@@ -146,6 +181,7 @@ struct Plan {
     int batch_kind = kCutScalar;
     int batch_grid = kGridDense;
     bool have_count = false;
+    bool count_pending = false;   // a force pass left no counts: made on demand
     int64_t npairs = 0;
     int quantities = 0;
     int64_t *host_small = nullptr;  // pinned: [0] pair count, [1] flags
@@ -189,7 +225,8 @@ nbl_status plan_system(const double origin[3], const double cell[9],
                        const double inv_cell[9], const uint8_t pbc[3], double cutoff,
                        SysDev &S, int64_t &ncells);
 nbl_status finish_batch(Batch &b, int grid_req);
-nbl_status upload_batch(Plan &p, const Batch &b, cudaStream_t st);
+nbl_status upload_batch(Plan &p, const Batch &b, cudaStream_t st, bool one_launch = false);
+void note_lists(Plan &p, const Batch &b, int64_t npairs, int64_t demand, int flags);
 nbl_status enqueue_count(Plan &p, const Batch &b, cudaStream_t st);
 nbl_status run_count(Plan &p, const Batch &b, cudaStream_t st, bool sync);
 nbl_status run_fill(Plan &p, const nbl_outputs &o, int64_t capacity, cudaStream_t st);

@@ -117,7 +117,10 @@ __device__ __forceinline__ void gather_one(const GatherArgs &a, int64_t s) {
         }
         float w32 = 0.f;
         if (S.cutoff_kind == kCutPerAtom) {
-            w32 = __double2float_rn(a.per_atom[at]);
+            const double radius = a.per_atom[at];
+            w32 = __double2float_rn(radius);
+            // (also for NaN and negative radii, whose squares mean nothing)
+            if (!(radius >= 0.0 && 2.0 * radius <= S.cutoff)) atomicOr(a.err, kNoteWideRadius);
         } else if (S.cutoff_kind == kCutPerType) {
             w32 = __int_as_float(a.types[at]);
         }
@@ -127,9 +130,17 @@ __device__ __forceinline__ void gather_one(const GatherArgs &a, int64_t s) {
                            (!S.pbc[2] && q[2] != 0);
         const int qp = quirk ? kImageWide : pack_image(q[0], q[1], q[2]);
         a.pos64[s] = make_double4(rel[0], rel[1], rel[2], __hiloint2double(qp, at));
-        a.pos32[s] = make_float4(__double2float_rn(rel[0]), __double2float_rn(rel[1]),
-                                 __double2float_rn(rel[2]), w32);
+        // FP32 copy: cell-relative, or (row passes) relative to the first cell of
+        // the atom's row along x, so that the row's cells share one frame
+        const double u = a.unroll ? (double)c[0] : 0.0;
+        a.pos32[s] = make_float4(__double2float_rn(rel[0] + u * S.bin[0][0]),
+                                 __double2float_rn(rel[1] + u * S.bin[0][1]),
+                                 __double2float_rn(rel[2] + u * S.bin[0][2]), w32);
         a.aux[s] = make_int4(at, q[0], q[1], q[2]);
+        if (a.hcell != nullptr) {
+            a.hcell[s] = make_int4(c[0], c[1], c[2], sysid);
+            a.inv[at] = (int32_t)s;
+        }
         amax = __double2float_ru(fmax(fabs(rel[0]), fmax(fabs(rel[1]), fabs(rel[2]))));
 
         const uint32_t key = a.keys[s];

@@ -156,9 +156,14 @@ __device__ __forceinline__ void emit_pair(const TraverseArgs &a, const Hot &H, c
 // (FILL = true, at offsets[i] on).  ALL5: all five outputs, no matrix.
 template <int KIND, bool FILL, bool ALL5>
 __device__ __forceinline__ void atom_row(const TraverseArgs &a, int64_t si) {
+    // after the row passes: only the rows that have no list
+    if (FILL && a.list != nullptr && !(*a.err & kErrNoList)) return;
     const int4 ai = a.aux[si];
     if (checked_fail(ai.x < 0 || ai.x >= a.natoms, a.err)) return;
     if (ai.x < a.i_lo || ai.x >= a.i_hi) return;
+    if (FILL && a.list != nullptr && 
+        a.counts[ai.x] <= (a.sys[a.hcell[si].w].list_cap - 1) * (a.list_wide ? 2 : 4))
+        return;
     int sys = 0;
     int32_t cc[3] = {0, 0, 0};
     if (!atom_home(a, si, ai.x, sys, cc)) return;
@@ -179,12 +184,13 @@ __device__ __forceinline__ void atom_row(const TraverseArgs &a, int64_t si) {
         slot = row0;
     }
     int cnt = 0;
-    const VisitDev *vt = a.visit + S.visit_base;
     const int nv = S.nvisit;
     for (int v = 0; v < nv; v++) {
-        const VisitDev &e = vt[v];
-        const int32_t d[3] = {e.d[0], e.d[1], e.d[2]};
-        int32_t cj[3], m[3];
+        int32_t d[3], cj[3], m[3];
+        float off32[3];
+        double off[3];
+        visit_at(a, S, v, d, off32);
+        visit_vector(a, S, v, off);
         if (!visit_cell(S, cc, d, cj, m)) continue;
         const int2 sl = cell_lookup(a, S, sys, cj[0], cj[1], cj[2]);
         if (checked_fail(sl.x < 0 || sl.y < sl.x || (long long)sl.y > a.natoms, a.err))
@@ -195,9 +201,9 @@ __device__ __forceinline__ void atom_row(const TraverseArgs &a, int64_t si) {
             if (sj == self) continue;
             const double4 pj = a.pos64[sj];
             const float tj = KIND == kCutPerType ? a.pos32[sj].w : 0.f;
-            if (!exact_inside<KIND>(H, a, pi, pj, e.off, wi, tj)) continue;
+            if (!exact_inside<KIND>(H, a, pi, pj, off, wi, tj)) continue;
             if (FILL)
-                emit_pair<ALL5>(a, H, ai, pi, pj, sj, e.off, m, slot++, row0);
+                emit_pair<ALL5>(a, H, ai, pi, pj, sj, off, m, slot++, row0);
             else
                 cnt++;
         }
@@ -216,6 +222,63 @@ __device__ __forceinline__ void atom_row(const TraverseArgs &a, int64_t si) {
     }
 }
 
+// One sorted atom's Lennard-Jones force and energy share, over the same walk.
+template <int KIND>
+__device__ __forceinline__ void atom_lj(const TraverseArgs &a, int64_t si) {
+    const double4 pi = a.pos64[si];
+    const int at = __double2loint(pi.w);
+    if (checked_fail(at < 0 || at >= a.natoms, a.err)) return;
+    if (at < a.i_lo || at >= a.i_hi) return;
+    double f[4] = {0.0, 0.0, 0.0, 0.0};
+    int sys = 0;
+    int32_t cc[3] = {0, 0, 0};
+    if (atom_home(a, si, at, sys, cc)) {
+        const SysDev &S = a.sys[sys];
+        Hot H;
+        H.cutoff_sq = S.cutoff_sq;
+        H.ncut = S.ncutoffs;
+        H.pt_base = S.pt_base;
+        const float wi = a.pos32[si].w;
+        const VisitDev *vt = a.visit + S.visit_base;
+        const int nv = S.nvisit;
+        for (int v = 0; v < nv; v++) {
+            const VisitDev &e = vt[v];
+            const int32_t d[3] = {e.d[0], e.d[1], e.d[2]};
+            int32_t cj[3], m[3];
+            if (!visit_cell(S, cc, d, cj, m)) continue;
+            const int2 sl = cell_lookup(a, S, sys, cj[0], cj[1], cj[2]);
+            if (checked_fail(sl.x < 0 || sl.y < sl.x || (long long)sl.y > a.natoms, a.err))
+                continue;
+            const int32_t self = (d[0] == 0 && d[1] == 0 && d[2] == 0) ? (int32_t)si : -1;
+            for (int32_t sj = sl.x; sj < sl.y; sj++) {
+                if (sj == self) continue;
+                const double4 pj = a.pos64[sj];
+                const double dx = dadd(dsub(pj.x, pi.x), e.off[0]);
+                const double dy = dadd(dsub(pj.y, pi.y), e.off[1]);
+                const double dz = dadd(dsub(pj.z, pi.z), e.off[2]);
+                const double r2 = dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz));
+                if (!(r2 < H.cutoff_sq)) continue;
+                if (KIND != kCutScalar &&
+                    !exact_inside<KIND>(H, a, pi, pj, e.off, wi,
+                                        KIND == kCutPerType ? a.pos32[sj].w : 0.f))
+                    continue;
+                lj_pair(a, dx, dy, dz, r2, f);
+            }
+        }
+    }
+    a.lj_force[3 * (int64_t)at + 0] = f[0];
+    a.lj_force[3 * (int64_t)at + 1] = f[1];
+    a.lj_force[3 * (int64_t)at + 2] = f[2];
+    a.lj_energy[at] = f[3];
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(kAtomThreads)
+k_atoms_lj(const __grid_constant__ TraverseArgs a) {
+    const int64_t si = (int64_t)blockIdx.x * kAtomThreads + threadIdx.x;
+    if (si < a.natoms) atom_lj<KIND>(a, si);
+}
+
 template <int KIND, bool FILL, bool ALL5>
 __global__ void __launch_bounds__(kAtomThreads)
 k_atoms(TraverseArgs a) {
@@ -232,7 +295,7 @@ TravKernel atoms_kernel(int kind) {
 
 cudaError_t launch_atoms(TravKernel k, const TraverseArgs &a, cudaStream_t st) {
     if (a.natoms <= 0) return cudaSuccess;
-    if (a.visit == nullptr || a.skeys == nullptr) return cudaErrorInvalidValue;
+    if (a.skeys == nullptr) return cudaErrorInvalidValue;
     const int64_t grid = (a.natoms + kAtomThreads - 1) / kAtomThreads;
     k<<<(unsigned)grid, kAtomThreads, 0, st>>>(a);
     count_launch();
@@ -240,6 +303,13 @@ cudaError_t launch_atoms(TravKernel k, const TraverseArgs &a, cudaStream_t st) {
 }
 
 }  // namespace
+
+cudaError_t launch_lj_atoms(int kind, const TraverseArgs &a, cudaStream_t st) {
+    const TravKernel k = kind == kCutPerAtom   ? k_atoms_lj<kCutPerAtom>
+                         : kind == kCutPerType ? k_atoms_lj<kCutPerType>
+                                               : k_atoms_lj<kCutScalar>;
+    return launch_atoms(k, a, st);
+}
 
 cudaError_t launch_count_atoms(int kind, const TraverseArgs &a, cudaStream_t st) {
     return launch_atoms(atoms_kernel<false, false>(kind), a, st);

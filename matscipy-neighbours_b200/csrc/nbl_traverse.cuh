@@ -4,9 +4,8 @@
 // them (nbl_trav_*.cu); everything here has internal linkage, so each unit
 // carries only the instantiations it launches.
 //
-// Shared memory is dynamic: a CTA holds one per-warp state block per warp
-// (plus, for the force sink, the warps' per-atom sums), sized by
-// count_smem_bytes / fill_smem_bytes below.
+// Shared memory is dynamic: a CTA holds one per-warp state block per warp,
+// sized by count_smem_bytes / fill_smem_bytes below.
 #pragma once
 
 #include <climits>
@@ -120,6 +119,47 @@ __device__ __forceinline__ SegVals seg_vals(const SegRec &g) {
     return v;
 }
 
+constexpr unsigned kNoLink = 0xffffffffu;
+
+// A list entry: sorted atom and visit, in one word where they fit (the visit
+// above the low `shift` bits), else (WIDE) in two.  Lists are made of 16-byte
+// groups.
+template <bool WIDE>
+struct Entry {
+    static constexpr int kPerGroup = WIDE ? 2 : 4;
+    using T = typename std::conditional<WIDE, uint2, unsigned>::type;
+    static __device__ __forceinline__ T make(int shift, int sj, int v) {
+        if constexpr (WIDE)
+            return make_uint2((unsigned)sj, (unsigned)v);
+        else
+            return (unsigned)sj | (unsigned)v << shift;
+    }
+    static __device__ __forceinline__ void get(int shift, T e, int &sj, int &v) {
+        if constexpr (WIDE) {
+            sj = (int)e.x;
+            v = (int)e.y;
+        } else {
+            sj = (int)(e & ((1u << shift) - 1u));
+            v = (int)(e >> shift);
+        }
+    }
+};
+
+// Links a new chunk at group `at`; returns its first group, -1 when there is
+// none left.
+__device__ __noinline__ long long list_grow(const TraverseArgs &a, long long at) {
+    const unsigned long long next =
+        (unsigned long long)a.list_chunks +
+        atomicAdd(a.mask_cursor, (unsigned long long)kListChunk);
+    if (next + kListChunk > (unsigned long long)a.list_cap) {
+        a.list[at] = make_uint4(kNoLink, kNoLink, 0u, 0u);
+        atomicOr(a.err, kErrNoList);
+        return -1;
+    }
+    a.list[at] = make_uint4((unsigned)next, (unsigned)(next >> 32), 0u, 0u);
+    return (long long)next;
+}
+
 template <bool FP32, int CAND>
 struct __align__(16) CountSmem {
     SegSmem sg;
@@ -138,8 +178,7 @@ constexpr int kPosTab = 640;     // pairs per window with a position table (fill
 static_assert(kRange <= 8192 && kITile <= 32,
               "position-table entries hold the candidate in 13 bits, the atom in 5");
 
-// Per-warp fill state, about 9.6 KB, so that five 4-warp CTAs fit an SM
-// (the force sink's sums live in a separate array of the force-sink kernel).
+// Per-warp fill state, about 9.6 KB, so that five 4-warp CTAs fit an SM.
 template <bool FP32>
 struct __align__(16) FillSmem {
     SegSmem sg;
@@ -157,10 +196,9 @@ struct __align__(16) FillSmem {
     uint8_t cand_seg[kCandTab];     // segment of each of the batch's first candidates
     int8_t ht[kITile];              // runs: each atom's home cell within the run
 };
-static_assert(5 * (4 * sizeof(FillSmem<true>) + 4 * 32 * 32 + 1024) <= 233472 &&
-                  5 * (4 * sizeof(FillSmem<false>) + 4 * 32 * 32 + 1024) <= 233472,
-              "five 4-warp fill CTAs per SM (force-sink sums included) fit the SM's "
-              "shared memory");
+static_assert(5 * (4 * sizeof(FillSmem<true>) + 1024) <= 233472 &&
+                  5 * (4 * sizeof(FillSmem<false>) + 1024) <= 233472,
+              "five 4-warp fill CTAs per SM fit the SM's shared memory");
 
 // Per-home-cell constants kept in registers.
 struct Hot {
@@ -230,6 +268,41 @@ __device__ __forceinline__ int2 cell_lookup(const TraverseArgs &a, const SysDev 
     const unsigned long long key =
         ((unsigned long long)sysid << kHashSysShift) | (unsigned long long)lin;
     return hash_find(a.hkey, a.hmask, a.table, key, a.err);
+}
+
+// Visited offset v of system S: cell offset and, as asked, its vector.
+__device__ __forceinline__ void visit_at(const TraverseArgs &a, const SysDev &S, int v, int d[3],
+                                         float *off32) {
+    if (S.visit_base >= 0) {
+        const VisitDev &e = a.visit[S.visit_base + v];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            d[k] = e.d[k];
+            off32[k] = e.off32[k];
+        }
+        return;
+    }
+    const int wx = 2 * S.nscan[0] + 1, wy = 2 * S.nscan[1] + 1, rest = v / wx;
+    d[0] = v % wx - S.nscan[0];
+    d[1] = rest % wy - S.nscan[1];
+    d[2] = rest / wy - S.nscan[2];
+    double o[3];
+    visit_offset(S, d, o);
+#pragma unroll
+    for (int k = 0; k < 3; k++) off32[k] = __double2float_rn(o[k]);
+}
+__device__ __forceinline__ void visit_vector(const TraverseArgs &a, const SysDev &S, int v,
+                                             double o[3]) {
+    if (S.visit_base >= 0) {
+        const VisitDev &e = a.visit[S.visit_base + v];
+        o[0] = e.off[0];
+        o[1] = e.off[1];
+        o[2] = e.off[2];
+        return;
+    }
+    const int wx = 2 * S.nscan[0] + 1, wy = 2 * S.nscan[1] + 1, rest = v / wx;
+    const int d[3] = {v % wx - S.nscan[0], rest % wy - S.nscan[1], rest / wy - S.nscan[2]};
+    visit_offset(S, d, o);
 }
 
 // Segment batch vb of a home cell: one lane per visited offset
@@ -507,6 +580,21 @@ __device__ __forceinline__ float3 run_frame32(const SysDev &S, int t) {
     visit_offset(S, d, o);
     return make_float3(__double2float_rn(o[0]), __double2float_rn(o[1]),
                        __double2float_rn(o[2]));
+}
+
+// One pair's force on atom i and energy share (lj_langevin_gpu.cu:59-74): U =
+// 4 eps ((sigma/r)^12 - (sigma/r)^6) cut at the list's cutoff, F_i = -24 eps s6
+// (2 s6 - 1) D / r^2, half of U per directed pair.
+__device__ __forceinline__ void lj_pair(const TraverseArgs &a, double dx, double dy, double dz,
+                                        double r2, double f[4]) {
+    const double ir2 = 1.0 / r2;
+    const double s2 = a.lj_sig2 * ir2;
+    const double s6 = s2 * s2 * s2;
+    const double coef = -a.lj_eps24 * ir2 * s6 * (2.0 * s6 - 1.0);
+    f[0] += coef * dx;
+    f[1] += coef * dy;
+    f[2] += coef * dz;
+    f[3] += 0.5 * a.lj_eps4 * (s6 * s6 - s6);
 }
 
 // FP32 thresholds for one (atom, candidate) pair.
@@ -1107,74 +1195,15 @@ __device__ __forceinline__ void store_pair(const FillSmem<FP32> &sm, const Trave
     }
 }
 
-// Force sink: one round of pairs, all 32 lanes.  Each active lane forms its
-// pair's Lennard-Jones force on atom i from the exact FP64 D (the reference's
-// operation order, as the stored D), U = 4 eps ((sigma/r)^12 - (sigma/r)^6)
-// cut at the list's cutoff, F_i = -24 eps s6 (2 s6 - 1) D / r^2 with
-// s6 = (sigma^2 / r^2)^3 (lj_langevin_gpu.cu:59-74 with eps = sigma = 1); the
-// lanes' forces and energy shares (1/2 U per directed pair) are summed per
-// atom (runs of equal i are contiguous) and the run's last lane adds them to
-// the tile's shared-memory sums.
-template <bool FP32, bool RUN>
-__device__ __forceinline__ void lj_round(const FillSmem<FP32> &sm, double (*facc)[4],
-                                         const TraverseArgs &a, const Hot &H, const PairWork &w,
-                                         int lane) {
-    const unsigned full = 0xffffffffu;
-    double f0 = 0.0, f1 = 0.0, f2 = 0.0, e = 0.0;
-    const int il = w.act ? w.il : -1;
-    if (w.act) {
-        const double4 pi = sm.i64[w.il];
-        const SegVals g = pair_seg_vals<FP32, RUN>(sm, a, H, w.seg, w.il);
-        const double dx = dadd(dsub(w.pj.x, pi.x), g.o0);
-        const double dy = dadd(dsub(w.pj.y, pi.y), g.o1);
-        const double dz = dadd(dsub(w.pj.z, pi.z), g.o2);
-        const double r2 = dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz));
-        const double ir2 = 1.0 / r2;
-        const double s2 = a.lj_sig2 * ir2;
-        const double s6 = s2 * s2 * s2;
-        const double coef = -a.lj_eps24 * ir2 * s6 * (2.0 * s6 - 1.0);
-        f0 = coef * dx;
-        f1 = coef * dy;
-        f2 = coef * dz;
-        e = 0.5 * a.lj_eps4 * (s6 * s6 - s6);
-    }
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const double t0 = __shfl_up_sync(full, f0, d);
-        const double t1 = __shfl_up_sync(full, f1, d);
-        const double t2 = __shfl_up_sync(full, f2, d);
-        const double t3 = __shfl_up_sync(full, e, d);
-        const int ii = __shfl_up_sync(full, il, d);
-        if (lane >= d && ii == il) {
-            f0 += t0;
-            f1 += t1;
-            f2 += t2;
-            e += t3;
-        }
-    }
-    const int inext = __shfl_down_sync(full, il, 1);
-    if (il >= 0 && (lane == 31 || inext != il)) {
-        facc[il][0] += f0;
-        facc[il][1] += f1;
-        facc[il][2] += f2;
-        facc[il][3] += e;
-    }
-    __syncwarp();
-}
-
-template <bool FP32, int KIND, bool LJ, bool ALL5, int WARPS, bool RUN>
+template <bool FP32, int KIND, bool ALL5, int WARPS, bool RUN>
 __global__ void __launch_bounds__(WARPS * 32, fill_min_blocks(WARPS))
 k_fill(TraverseArgs a) {
     constexpr int kCand = FillTile<FP32>::kCand;
     constexpr int kWarps = WARPS;
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     FillSmem<FP32> *smem = reinterpret_cast<FillSmem<FP32> *>(dyn_smem);
-    // force sink: each warp's tile force and energy sums, after the warps' state
-    double(*facc_all)[4] =
-        reinterpret_cast<double(*)[4]>(dyn_smem + sizeof(FillSmem<FP32>) * WARPS);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     FillSmem<FP32> &sm = smem[warp];
-    double(*facc)[4] = facc_all + (LJ ? warp * kITile : 0);
     const unsigned full = 0xffffffffu;
     const int nitems = *a.n_items;
     const int gwarp = blockIdx.x * kWarps + warp, nwarps = gridDim.x * kWarps;
@@ -1212,7 +1241,6 @@ k_fill(TraverseArgs a) {
                     cp_async16(&sm.iaux[lane], &a.aux[ib + lane]);
                     sm.isi[lane] = ib + lane;
                     sm.ht[lane] = (int8_t)t_l;
-                    if (LJ) facc[lane][0] = facc[lane][1] = facc[lane][2] = facc[lane][3] = 0.0;
                 }
                 off_pending = true;
             } else {
@@ -1235,7 +1263,6 @@ k_fill(TraverseArgs a) {
                     sm.icur[c2] = checked_fail(ax.x >= a.natoms, a.err)
                                       ? 0ll
                                       : (long long)a.offsets[ax.x];
-                    if (LJ) facc[c2][0] = facc[c2][1] = facc[c2][2] = facc[c2][3] = 0.0;
                 }
                 __syncwarp();
             }
@@ -1385,10 +1412,7 @@ k_fill(TraverseArgs a) {
                             const PairWork nxt = fetch_pair<FP32>(sm, a, nseg, nchunks, nw,
                                                                   nch, inv_nch, kr, a0, carry,
                                                                   P0 + 32 + lane, tab);
-                            if (LJ)
-                                lj_round<FP32, RUN>(sm, facc, a, H, cur, lane);
-                            else
-                                store_pair<FP32, ALL5, RUN>(sm, a, H, cur, !cap_ok);
+                            store_pair<FP32, ALL5, RUN>(sm, a, H, cur, !cap_ok);
                             cur = nxt;
                         }
                         __syncwarp();
@@ -1414,12 +1438,6 @@ k_fill(TraverseArgs a) {
                     a.mat_count[ax] = (int32_t)deg;
                     if (deg > a.mat_k) atomicOr(a.mat_overflow, 1);
                 }
-                if (LJ) {
-                    a.lj_force[3 * (long long)ax + 0] = facc[lane][0];
-                    a.lj_force[3 * (long long)ax + 1] = facc[lane][1];
-                    a.lj_force[3 * (long long)ax + 2] = facc[lane][2];
-                    a.lj_energy[ax] = facc[lane][3];
-                }
             }
             __syncwarp();
         } while (0);
@@ -1433,9 +1451,8 @@ constexpr size_t count_smem_bytes(int warps) {
     return sizeof(CountSmem<FP32, CAND>) * (size_t)warps;
 }
 template <bool FP32>
-constexpr size_t fill_smem_bytes(int warps, bool lj) {
-    return sizeof(FillSmem<FP32>) * (size_t)warps +
-           (lj ? sizeof(double) * 4 * kITile * (size_t)warps : sizeof(double) * 4);
+constexpr size_t fill_smem_bytes(int warps) {
+    return sizeof(FillSmem<FP32>) * (size_t)warps;
 }
 
 using TravKernel = void (*)(TraverseArgs);
