@@ -280,11 +280,21 @@ int64_t ListPlan::cap(double m) const {
     return (int64_t)std::ceil(e / (wide ? 2.0 : 4.0)) + 1;  // and the link
 }
 
+// Whether the atoms are ordered by counting them into cells (cell_order) instead
+// of a radix sort of their cell keys: where the keys number the table's entries
+// (not Morton codes) and the table is within the size the automatic grid choice
+// allows, so that scanning it stays small beside the atoms.
+static bool counted_cells(const Batch &b) {
+    return b.grid != kGridMorton &&
+           b.table_size <= std::max<int64_t>(int64_t(1) << 20, 8 * b.natoms);
+}
+
 // Carve the per-call buffers out of the plan's workspace.
 static nbl_status layout_workspace(Plan &p, const Batch &b) {
     const int64_t N = b.natoms;
     const int64_t nsys = (int64_t)b.sys.size();
-    const int64_t hist = radix_hist_elems(std::max<int64_t>(N, 1));
+    const bool counted = counted_cells(b);
+    const int64_t hist = counted ? 0 : radix_hist_elems(std::max<int64_t>(N, 1));
     Layout L;
     Bufs &B = p.bufs;
     size_t o_pos = b.pos_on_device ? 0 : L.add(sizeof(double) * 3 * N);
@@ -304,7 +314,9 @@ static nbl_status layout_workspace(Plan &p, const Batch &b) {
     size_t o_vals2 = L.add(sizeof(int32_t) * N);
     size_t o_hist = L.add(sizeof(int32_t) * hist);
     size_t o_hscan = L.add(sizeof(int32_t) * hist);
-    size_t o_sscr32 = L.add(sizeof(int32_t) * scan_scratch_elems(hist));
+    size_t o_sscr32 =
+        L.add(sizeof(int32_t) * scan_scratch_elems(counted ? b.table_size : hist));
+    size_t o_cells = counted ? L.add(sizeof(int32_t) * b.table_size) : 0;
     size_t o_sscr64 = L.add(sizeof(int64_t) * scan_scratch_elems(N + 1));
     size_t o_table = L.add(sizeof(int2) * b.table_size);
     size_t o_hkey = b.grid == kGridHashed ? L.add(sizeof(unsigned long long) * b.table_size) : 0;
@@ -360,6 +372,7 @@ static nbl_status layout_workspace(Plan &p, const Batch &b) {
     B.hist_scan = (int32_t *)at(o_hscan);
     B.scan32 = (int32_t *)at(o_sscr32);
     B.scan64 = (int64_t *)at(o_sscr64);
+    B.cell_count = counted ? (int32_t *)at(o_cells) : nullptr;
     B.table = (int2 *)at(o_table);
     B.hkey = b.grid == kGridHashed ? (unsigned long long *)at(o_hkey) : nullptr;
     B.pos64 = (double4 *)at(o_pos64);
@@ -508,7 +521,7 @@ static int tile_of(const Plan &p, const Batch &b) {
 // cells stands in for it.  Measured on 200,000-atom uniform gases (count +
 // fill): 2.7x faster at 0.25 atoms per cell (1.1 per occupied cell), 2.0x at
 // 0.5 (1.3), 1.35x at 1 (1.6), even at 2 (2.3), slower above; even on a slab
-// of 2 atoms per occupied cell.  The force pass has its own rule (lj_atom_mode).
+// of 2 atoms per occupied cell.
 static bool atom_mode(const Plan &p, const Batch &b) {
     if (p.atom_threads < 0 || p.bufs.visit == nullptr) return false;
     if (p.atom_threads > 0) return true;
@@ -527,16 +540,6 @@ static bool sparse_grid(const Plan &p, const Batch &b) {
     double cells = 0.0;
     for (int64_t n : b.ncells) cells += (double)n;
     return (double)b.natoms < kSparseAtoms * cells;
-}
-
-// Whether the Lennard-Jones pass runs one thread per atom: it needs no second
-// walk to write pairs, so the line lies higher than the list's.
-static bool lj_atom_mode(const Plan &p, const Batch &b) {
-    if (p.atom_threads < 0 || p.bufs.visit == nullptr) return false;
-    if (p.atom_threads > 0) return true;
-    double cells = 0.0;
-    for (int64_t n : b.ncells) cells += (double)n;
-    return (double)b.natoms < kLjAtomsPerCell * cells;
 }
 
 // Size the workspace for a batch and copy its inputs and host tables in.
@@ -635,6 +638,8 @@ static void bin_args(const Plan &p, const Batch &b, BinArgs &ba) {
     ba.natoms = b.natoms;
     ba.keys = B.keys;
     ba.vals = B.vals;
+    ba.cell_count = nullptr;
+    ba.crowded = 0;
     ba.hkey = B.hkey;
     ba.hmask = (unsigned long long)(b.table_size - 1);
     ba.err = B.small + 1;
@@ -653,6 +658,7 @@ static void gather_args(const Plan &p, const Batch &b, const uint32_t *skeys,
     ga.natoms = b.natoms;
     ga.keys = skeys;
     ga.vals = svals;
+    ga.skeys = nullptr;
     ga.table = B.table;
     ga.pos64 = B.pos64;
     ga.pos32 = B.pos32;
@@ -664,6 +670,9 @@ static void gather_args(const Plan &p, const Batch &b, const uint32_t *skeys,
     ga.amax = B.amax;
     ga.home = B.home;
     ga.n_home = B.small + 0;
+    ga.items = nullptr;
+    ga.n_items = B.small + 3;
+    ga.itile = 0;
 }
 
 static void traverse_args(Plan &p, const Batch &b, bool atoms, int max_run) {
@@ -729,28 +738,48 @@ static nbl_status enqueue_build(Plan &p, const Batch &b, bool atoms, int max_run
     Bufs &B = p.bufs;
     const int64_t N = b.natoms;
     const int nsys = (int)b.sys.size();
-    NBL_CUDA(launch_init(B.sys, nsys, B.visit, B.small, B.table, b.table_size, B.amax,
+    NBL_CUDA(launch_init(B.sys, nsys, B.visit, B.small, B.table, B.cell_count, b.table_size, B.amax,
                          b.grid == kGridHashed ? B.hkey : nullptr, p.num_sms, st),
              "k_init");
     BinArgs ba;
     bin_args(p, b, ba);
+    const bool counted = B.cell_count != nullptr;
+    ba.cell_count = B.cell_count;
+    // (matching a warp's cells: 28.7 -> 13.9 us on 4,096 small systems of some 30
+    // atoms per cell, 12.2 -> 16.0 us on the dense bulk at 10)
+    ba.crowded = N >= 16 * b.table_size ? 1 : 0;
     {
         StageRange r("nbl.bin");
         NBL_CUDA(launch_bin(ba, st), "k_bin");
     }
     bool in_alt = false;
+    GatherArgs ga;
+    const bool items = !atoms && !p.sparse;  // passes by atoms need no work items
     {
         StageRange r("nbl.sort");
-        NBL_CUDA(radix_sort_pairs(B.keys, B.vals, B.keys2, B.vals2, N, b.key_bits, B.hist,
-                                  B.hist_scan, B.scan32, st, &in_alt),
-                 "radix sort");
+        if (counted) {
+            NBL_CUDA(cell_order(B.keys, B.vals, B.cell_count, N, b.table_size, B.scan32,
+                                B.small + 7, B.table, B.vals2, st),
+                     "cell order");
+            gather_args(p, b, B.keys, B.vals2, ga);
+            ga.skeys = B.keys2;
+            in_alt = true;
+            if (items && max_run == 1) {  // one cell per item: the gather makes them
+                ga.items = B.items;
+                ga.itile = tile_of(p, b);
+                ga.home = nullptr;
+            }
+        } else {
+            NBL_CUDA(radix_sort_pairs(B.keys, B.vals, B.keys2, B.vals2, N, b.key_bits, B.hist,
+                                      B.hist_scan, B.scan32, st, &in_alt),
+                     "radix sort");
+            gather_args(p, b, in_alt ? B.keys2 : B.keys, in_alt ? B.vals2 : B.vals, ga);
+        }
     }
-    GatherArgs ga;
-    gather_args(p, b, in_alt ? B.keys2 : B.keys, in_alt ? B.vals2 : B.vals, ga);
     {
         StageRange r("nbl.gather");
         NBL_CUDA(launch_gather(ga, st), "k_gather");
-        if (!atoms && !p.sparse)  // passes by atoms and sparse counts need no work items
+        if (items && ga.items == nullptr)
             NBL_CUDA(launch_tiles(B.home, ga.n_home, B.table, B.sys, B.items, B.small + 3, N,
                                   p.num_sms, tile_of(p, b), max_run, st),
                      "k_tiles");
@@ -783,7 +812,7 @@ static nbl_status enqueue_count_pass(Plan &p, bool ticket_ready, cudaStream_t st
     }
     {
         StageRange r("nbl.scan");
-        NBL_CUDA(exclusive_scan_i32_i64(B.counts, N, B.offsets, B.scan64, st), "scan");
+        NBL_CUDA(exclusive_scan_i32_i64(B.counts, N, B.offsets, B.scan64, st, B.small + 7), "scan");
         if (p.rows) NBL_CUDA(launch_row_marks(p.targs, st), "row marks");
     }
     return NBL_SUCCESS;
@@ -1462,7 +1491,7 @@ nbl_status nbl_lj_forces(nbl_plan *plan, const nbl_request *req, double epsilon,
     Plan &p = plan->p;
     st = upload_batch(p, b, cs, false);
     if (st != NBL_SUCCESS) return st;
-    const bool atoms = lj_atom_mode(p, b);
+    const bool atoms = p.rows || p.atom_threads > 0;
     st = enqueue_build(p, b, atoms, 1, cs);
     if (st != NBL_SUCCESS) return st;
     p.have_count = true;

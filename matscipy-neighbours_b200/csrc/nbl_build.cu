@@ -6,15 +6,20 @@
 //               visited cell offsets' vectors (reference order) per system
 //   k_bin       per atom: raw cell (reference arithmetic), fold, cell key;
 //               hashed grid: insert the cell into the open-addressing table
-//   radix sort  (nbl_sort.cu) stable by cell key -> cell-sorted atom order
+//   cell order  (nbl_sort.cu) scan of the cells' counts, atoms into their cell's
+//               slice; or (Morton keys, huge tables) a stable radix sort by key
 //   k_gather    per sorted atom: bin-relative position (FP64, reference
 //               arithmetic), its FP32 copy, image indices, cell slices,
 //               occupied-cell work list
+//               (and the work items, where they hold one cell each)
 //   k_tiles     occupied cells -> work items (home cell x i-tile of <= 32
 //               atoms, or runs of sparse cells along x)
-//   k_count     per work item: neighbour counts per atom, hit words
+//   count       neighbour lists and counts (nbl_trav_list.cu, nbl_rows.cu); or,
+//               where the configuration asks for the warp passes, k_count: per
+//               work item, neighbour counts per atom and hit words
 //   scan        (nbl_sort.cu) counts -> row offsets, total pair count
-//   k_fill      per work item: writes i, j, D, d, S (or feeds a force sink)
+//   fill        k_rows_fill (nbl_rows.cu): the lists as i, j, D, d, S in output
+//               order; or k_fill, per work item, from the hit words
 // A small system's count phase (init to scan) can instead be one launch
 // (nbl_small.cu).
 //
@@ -105,7 +110,8 @@ cudaError_t launch_tiles(const HomeCell *home, const int *n_home, const int2 *ta
 // the hash slots) and the per-system maxima.
 __global__ void __launch_bounds__(256)
 k_init(const SysDev *__restrict__ sys, int nsys, VisitDev *__restrict__ visit,
-       int *__restrict__ small, int2 *__restrict__ table, int64_t ntable,
+       int *__restrict__ small, int2 *__restrict__ table,
+       int32_t *__restrict__ cell_count, int64_t ntable,
        float *__restrict__ amax, unsigned long long *__restrict__ hkey) {
     if (visit != nullptr && (int)blockIdx.x < nsys)
         visit_fill(sys[blockIdx.x], visit, threadIdx.x, blockDim.x);
@@ -113,20 +119,24 @@ k_init(const SysDev *__restrict__ sys, int nsys, VisitDev *__restrict__ visit,
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
     if (t0 < 8) small[t0] = 0;
     for (int64_t i = t0; i < ntable; i += step) {
-        table[i] = make_int2(0, 0);
+        if (cell_count != nullptr)
+            cell_count[i] = 0;  // (the slices are all written later)
+        else
+            table[i] = make_int2(0, 0);
         if (hkey != nullptr) hkey[i] = kHashEmpty;
     }
     for (int64_t i = t0; i < nsys; i += step) amax[i] = 0.f;
 }
 
 cudaError_t launch_init(const SysDev *sys, int nsys, VisitDev *visit, int *small, int2 *table,
-                        int64_t ntable, float *amax, unsigned long long *hkey, int num_sms,
+                        int32_t *cell_count, int64_t ntable, float *amax, unsigned long long *hkey, int num_sms,
                         cudaStream_t st) {
     const int64_t work = std::max<int64_t>(ntable, nsys);
     int64_t blocks = std::min<int64_t>((work + 255) / 256, (int64_t)num_sms * 8);
     blocks = std::max<int64_t>(blocks, visit != nullptr ? nsys : 1);
     blocks = std::max<int64_t>(blocks, 1);
-    k_init<<<(unsigned)blocks, 256, 0, st>>>(sys, nsys, visit, small, table, ntable, amax, hkey);
+    k_init<<<(unsigned)blocks, 256, 0, st>>>(sys, nsys, visit, small, table, cell_count, ntable, amax,
+                                         hkey);
     count_launch();
     return cudaGetLastError();
 }

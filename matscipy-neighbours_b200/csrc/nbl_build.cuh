@@ -20,7 +20,9 @@ struct BinArgs {
     const double *positions;  // [3*natoms], concatenated systems
     int64_t natoms;
     uint32_t *keys;
-    int32_t *vals;
+    int32_t *vals;            // the atom's index, or (cell_count) its arrival in its cell
+    int32_t *cell_count;      // [cells], zeroed, or null
+    int crowded;              // many atoms per cell: a warp's atoms of a cell count together
     unsigned long long *hkey;
     unsigned long long hmask;
     int *err;
@@ -35,8 +37,9 @@ struct GatherArgs {
     const double *per_atom;   // [natoms] or null
     const int32_t *types;     // [natoms] or null
     int64_t natoms;
-    const uint32_t *keys;     // sorted
-    const int32_t *vals;      // sorted: global atom index
+    const uint32_t *keys;     // sorted; per atom with skeys
+    const int32_t *vals;      // sorted: global atom index; with skeys by cell, any order within
+    uint32_t *skeys;          // non-null: written sorted, the table holds the slices already
     int2 *table;
     double4 *pos64;
     float4 *pos32;
@@ -46,8 +49,11 @@ struct GatherArgs {
     int unroll;               // pos32 unrolled along x (the row passes' frame)
     int *err;
     float *amax;              // [nsys], zeroed
-    HomeCell *home;
+    HomeCell *home;           // occupied cells, or null
     int *n_home;              // zeroed
+    WorkItem *items;          // work items of up to itile atoms (with skeys), or null
+    int *n_items;             // zeroed
+    int itile;
 };
 
 struct TraverseArgs {
@@ -198,9 +204,11 @@ cudaError_t launch_count_small(bool fp32, int kind, const SmallCountArgs &a, int
                                cudaStream_t st);
 
 // Start of a count phase in one launch: zero the 8-int flag block, the cell
-// table (ntable int2) and the per-system maxima, mark every hash slot empty
+// table (ntable int2) or, if not null, the cell counts (ntable ints), and the
+// per-system maxima, mark every hash slot empty
 // (hkey != NULL), and fill the systems' visit tables (visit != NULL).
 cudaError_t launch_init(const SysDev *sys, int nsys, VisitDev *visit, int *small, int2 *table,
+                        int32_t *cell_count,
                         int64_t ntable, float *amax, unsigned long long *hkey, int num_sms,
                         cudaStream_t st);
 // Work items: each occupied cell cut into tiles of `itile` (<= 32) atoms, or

@@ -55,6 +55,7 @@ struct Bufs {
     float *pt32 = nullptr;
     uint32_t *keys = nullptr, *keys2 = nullptr;
     int32_t *vals = nullptr, *vals2 = nullptr;
+    int32_t *cell_count = nullptr;  // atoms per cell (counted_cells), or null
     int32_t *hist = nullptr, *hist_scan = nullptr, *scan32 = nullptr;
     int64_t *scan64 = nullptr;
     int2 *table = nullptr;
@@ -108,9 +109,6 @@ constexpr int64_t kMarkAtoms = 131072;
 // Atoms per occupied cell below which the count takes one thread per atom
 // (k_rows_count against k_count_list: 84 / 214 us at 2.3, 674 / 490 at 10).
 constexpr double kSparseAtoms = 4.0;
-
-// Atoms per cell below which the Lennard-Jones pass takes one thread per atom.
-constexpr double kLjAtomsPerCell = 1e9;
 
 // Everything that shapes the count phase's launches on a plan: when two
 // consecutive single calls have the same key, the second captures the count

@@ -11,8 +11,17 @@ namespace nbl {
 int64_t scan_scratch_elems(int64_t n);
 
 // out[k] = sum(in[0..k)), k < n, and out[n] = sum(in[0..n)).
+// With a ticket (one zeroed int, zero again afterwards) the scan of a larger
+// input takes two launches instead of three or more.
 cudaError_t exclusive_scan_i32_i64(const int32_t *in, int64_t n, int64_t *out,
-                                   int64_t *scratch, cudaStream_t st);
+                                   int64_t *scratch, cudaStream_t st, int *ticket = nullptr);
+
+// Cell slices from the cells' counts, and the atoms' order by cell, within a
+// cell by arrival (the gather ranks them by index).  carry holds
+// scan_scratch_elems(ncells) values; ticket as above.
+cudaError_t cell_order(const uint32_t *keys, const int32_t *arrival, const int32_t *count,
+                       int64_t natoms, int64_t ncells, int32_t *carry, int *ticket, int2 *table,
+                       int32_t *order, cudaStream_t st);
 // out[k] = sum(in[0..k)), k < n.
 cudaError_t exclusive_scan_i32_i32(const int32_t *in, int64_t n, int32_t *out,
                                    int32_t *scratch, cudaStream_t st);

@@ -71,13 +71,25 @@ __device__ __forceinline__ void bin_one(const BinArgs &a, int64_t t) {
         key = (uint32_t)(S.key_base + lin);
     }
     a.keys[t] = key;
-    a.vals[t] = (int32_t)t;
+    if (a.cell_count != nullptr && a.crowded) {  // one atomic per cell and warp
+        const unsigned peers = __match_any_sync(__activemask(), key);
+        const int lead = __ffs(peers) - 1;
+        int first = 0;
+        if ((int)(threadIdx.x & 31) == lead)
+            first = atomicAdd(a.cell_count + key, __popc(peers));
+        a.vals[t] = __shfl_sync(peers, first, lead) + __popc(peers & lanemask_lt());
+    } else if (a.cell_count != nullptr) {
+        a.vals[t] = atomicAdd(a.cell_count + key, 1);
+    } else {
+        a.vals[t] = (int32_t)t;
+    }
 }
 
 // Sorted atom s (valid: s < natoms); every lane of the warp takes part (the
 // per-system maxima and the occupied-cell list are aggregated per warp).
 __device__ __forceinline__ void gather_one(const GatherArgs &a, int64_t s) {
     const bool valid = s < a.natoms;
+    int2 seg = make_int2(0, 0);
     const unsigned full = 0xffffffffu;
     bool start = false;
     int sysid = 0;
@@ -86,6 +98,18 @@ __device__ __forceinline__ void gather_one(const GatherArgs &a, int64_t s) {
     float amax = 0.f;
     if (valid) {
         const int32_t at = a.vals[s];
+        uint32_t key;
+        if (a.skeys != nullptr) {  // the atom's rank in its cell, by index
+            key = a.keys[at];
+            seg = a.table[key];
+            int rank = 0;
+#pragma unroll 4
+            for (int q = seg.x; q < seg.y; q++) rank += a.vals[q] < at ? 1 : 0;
+            s = seg.x + rank;
+            a.skeys[s] = key;
+        } else {
+            key = a.keys[s];
+        }
         sysid = a.nsys > 1 ? sys_of(a.sys_atom_base, a.nsys, at) : 0;
         const SysDev &S = a.sys[sysid];
         const double r[3] = {a.positions[3 * (int64_t)at + 0],
@@ -143,14 +167,17 @@ __device__ __forceinline__ void gather_one(const GatherArgs &a, int64_t s) {
         }
         amax = __double2float_ru(fmax(fabs(rel[0]), fmax(fabs(rel[1]), fabs(rel[2]))));
 
-        const uint32_t key = a.keys[s];
         const int64_t lin = (int64_t)c[0] +
                             (int64_t)S.n[0] * ((int64_t)c[1] + (int64_t)S.n[1] * c[2]);
         tidx = (a.grid == kGridMorton) ? (uint32_t)(S.cell_base + lin) : key;
-        start = (s == 0) || (a.keys[s - 1] != key);
-        const bool end = (s == a.natoms - 1) || (a.keys[s + 1] != key);
-        if (start) a.table[tidx].x = (int32_t)s;
-        if (end) a.table[tidx].y = (int32_t)(s + 1);
+        if (a.skeys != nullptr) {
+            start = s == seg.x;
+        } else {
+            start = (s == 0) || (a.keys[s - 1] != key);
+            const bool end = (s == a.natoms - 1) || (a.keys[s + 1] != key);
+            if (start) a.table[tidx].x = (int32_t)s;
+            if (end) a.table[tidx].y = (int32_t)(s + 1);
+        }
     }
     // Per-system max |rel| (non-negative floats order like their bit patterns):
     // one atomic per warp when the warp lies inside one system, else per lane.
@@ -174,7 +201,7 @@ __device__ __forceinline__ void gather_one(const GatherArgs &a, int64_t s) {
         int base = 0;
         if (lane == __ffs(m) - 1) base = atomicAdd(a.n_home, __popc(m));
         base = __shfl_sync(full, base, __ffs(m) - 1);
-        if (start) {
+        if (start && a.home != nullptr) {
             HomeCell h;
             h.tidx = (int32_t)tidx;
             h.sys = sysid;
@@ -183,6 +210,30 @@ __device__ __forceinline__ void gather_one(const GatherArgs &a, int64_t s) {
             h.c[2] = c[2];
             h.pad = 0;
             a.home[base + __popc(m & lanemask_lt())] = h;
+        }
+        if (a.items != nullptr) {  // the cell's work items (tiles_one, one cell each)
+            const int nt = start ? (seg.y - seg.x + a.itile - 1) / a.itile : 0;
+            int incl = nt;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int o = __shfl_up_sync(full, incl, d);
+                if (lane >= d) incl += o;
+            }
+            int first = 0;
+            if (lane == 31) first = atomicAdd(a.n_items, incl);
+            first = __shfl_sync(full, first, 31) + incl - nt;
+            for (int t = 0; t < nt; t++) {
+                WorkItem w;
+                w.c[0] = c[0];
+                w.c[1] = c[1];
+                w.c[2] = c[2];
+                w.sys = sysid;
+                w.ib = seg.x + a.itile * t;
+                w.nt = min(a.itile, seg.y - w.ib);
+                w.tidx = (int32_t)tidx;
+                w.run = 1;
+                a.items[first + t] = w;
+            }
         }
     }
 }
