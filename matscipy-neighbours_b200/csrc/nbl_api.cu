@@ -250,8 +250,11 @@ static double list_entries(double m) { return 1.1 * m + 4.0 * std::sqrt(m) + 4.0
 // and more, for chained chunks.
 static ListPlan plan_lists(const Plan &p, const Batch &b) {
     ListPlan lp;
-    const bool known = p.list_natoms == b.natoms && p.list_table == b.table_size;
-    const double scale = known ? p.list_scale : 1.0;
+    const bool known =
+        !p.forces && p.list_natoms == b.natoms && p.list_table == b.table_size;
+    // (a force pass writes no lists: should the list be asked for afterwards, most
+    // rows run out of room and the thread-per-atom fill writes them)
+    const double scale = p.forces ? 0.0 : known ? p.list_scale : 1.0;
     int max_visit = 0;
     for (const SysDev &S : b.sys) max_visit = std::max(max_visit, S.nvisit);
     lp.shift = 32 - bits_for((uint64_t)std::max(max_visit - 1, 1));
@@ -543,11 +546,13 @@ static bool sparse_grid(const Plan &p, const Batch &b) {
 }
 
 // Size the workspace for a batch and copy its inputs and host tables in.
-nbl_status upload_batch(Plan &p, const Batch &b, cudaStream_t st, bool one_launch) {
+nbl_status upload_batch(Plan &p, const Batch &b, cudaStream_t st, CountUse use) {
     // the row passes, unless the one-launch count phase or the launch
-    // configuration asks for the warp passes or the thread-per-atom passes
-    p.rows = !one_launch && p.atom_threads == 0 && p.max_run == 0;
-    p.sparse = p.rows && (!b.fp32 || sparse_grid(p, b));
+    // configuration asks for the warp passes or the thread-per-atom passes; a
+    // force pass walks as the sparse count does
+    p.forces = use == kUseForces;
+    p.rows = p.forces || (use == kUseLists && p.atom_threads == 0 && p.max_run == 0);
+    p.sparse = p.forces || (p.rows && (!b.fp32 || sparse_grid(p, b)));
     p.cand_atom = candidates_per_atom(b);
     nbl_status s = layout_workspace(p, b);
     if (s != NBL_SUCCESS) return s;
@@ -965,7 +970,7 @@ static bool capture_count(Plan &p, const Batch &b, const CountKey &k) {
 
 nbl_status run_count(Plan &p, const Batch &b, cudaStream_t st, bool sync) {
     const bool small = sync && small_path(p, b);
-    nbl_status s = upload_batch(p, b, st, small);
+    nbl_status s = upload_batch(p, b, st, small ? kUseOneLaunch : kUseLists);
     if (s != NBL_SUCCESS) return s;
     // Single calls: replay the captured count phase while the launch key
     // repeats (captured on the second call with the same key); a small
@@ -1489,10 +1494,9 @@ nbl_status nbl_lj_forces(nbl_plan *plan, const nbl_request *req, double epsilon,
     if (!g.ok) return set_error(NBL_ERROR_CUDA, "cannot select device %d", plan->p.device);
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
     Plan &p = plan->p;
-    st = upload_batch(p, b, cs, false);
+    st = upload_batch(p, b, cs, kUseForces);
     if (st != NBL_SUCCESS) return st;
-    const bool atoms = p.rows || p.atom_threads > 0;
-    st = enqueue_build(p, b, atoms, 1, cs);
+    st = enqueue_build(p, b, false, 1, cs);
     if (st != NBL_SUCCESS) return st;
     p.have_count = true;
     p.count_pending = true;
@@ -1501,16 +1505,12 @@ nbl_status nbl_lj_forces(nbl_plan *plan, const nbl_request *req, double epsilon,
         return NBL_SUCCESS;
     }
     TraverseArgs ta = p.targs;
-    ta.item_next = p.fill_tickets ? p.bufs.small + 6 : nullptr;
-    ta.ticket_ready = 1;  // k_init cleared the ticket
     ta.lj_force = forces;
     ta.lj_energy = p.bufs.lj_part;
     ta.lj_eps4 = 4.0 * epsilon;
     ta.lj_eps24 = 24.0 * epsilon;
     ta.lj_sig2 = sigma * sigma;
-    NBL_CUDA(atoms ? launch_lj_atoms(p.batch_kind, ta, cs)
-                   : launch_lj_items(p.batch_kind, ta, p.num_sms, cs),
-             "force pass");
+    NBL_CUDA(launch_lj_atoms(p.batch_kind, ta, cs), "force pass");
     NBL_CUDA(launch_lj_energy(p.bufs.lj_part, b.natoms, p.bufs.lj_part + b.natoms, energy,
                               cs),
              "energy");

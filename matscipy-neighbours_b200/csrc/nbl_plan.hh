@@ -123,6 +123,9 @@ struct CountKey {
     bool operator==(const CountKey &o) const { return std::memcmp(this, &o, sizeof(*this)) == 0; }
 };
 
+// What a batch is uploaded for.
+enum CountUse { kUseLists, kUseOneLaunch, kUseForces };
+
 struct Plan {
     int device = 0;
     int num_sms = 148;
@@ -166,6 +169,7 @@ struct Plan {
     // found: chained entries, pairs against the density's estimate.
     bool rows = false;
     double cand_atom = 0.0;   // atoms of the cells that an atom visits, on average
+    bool forces = false;      // a force pass: no lists planned
     bool sparse = false;      // with one thread per atom in the count
     bool lists_short = true;  // some row may have no list (kErrNoList)
     int64_t list_natoms = -1, list_table = -1, list_hint = 0;
@@ -223,7 +227,7 @@ nbl_status plan_system(const double origin[3], const double cell[9],
                        const double inv_cell[9], const uint8_t pbc[3], double cutoff,
                        SysDev &S, int64_t &ncells);
 nbl_status finish_batch(Batch &b, int grid_req);
-nbl_status upload_batch(Plan &p, const Batch &b, cudaStream_t st, bool one_launch = false);
+nbl_status upload_batch(Plan &p, const Batch &b, cudaStream_t st, CountUse use = kUseLists);
 void note_lists(Plan &p, const Batch &b, int64_t npairs, int64_t demand, int flags);
 nbl_status enqueue_count(Plan &p, const Batch &b, cudaStream_t st);
 nbl_status run_count(Plan &p, const Batch &b, cudaStream_t st, bool sync);

@@ -117,6 +117,25 @@ __device__ __forceinline__ bool fold_axis(int &x, int n, int periodic, int &m) {
     return true;
 }
 
+// Atom A.si's filter record and thresholds; its cell and system are set.
+template <bool FP32>
+__device__ __forceinline__ void row_thresholds(const TraverseArgs &a, const SysDev &S, RowAtom &A) {
+    A.p32 = a.pos32[A.si];
+    A.H.lo_rc = A.H.hi_rc = A.H.band = 0.f;
+    if (FP32) {
+        const double ext = (double)S.n[0] *
+                           fmax(fabs(S.bin[0][0]), fmax(fabs(S.bin[0][1]), fabs(S.bin[0][2])));
+        const double band =
+            guard_band(2.0 * ((double)a.amax[A.sys] + ext) + S.off_max + ext, S.cutoff);
+        A.H.lo_rc = __double2float_rd(S.cutoff_sq - band);
+        A.H.hi_rc = __double2float_ru(S.cutoff_sq + band);
+        A.H.band = __double2float_ru(band);
+    }
+    A.H.cutoff_sq = S.cutoff_sq;
+    A.H.ncut = S.ncutoffs;
+    A.H.pt_base = S.pt_base;
+}
+
 // A guard-band candidate, decided exactly.
 template <int KIND>
 __device__ __noinline__ bool row_exact(const TraverseArgs &a, const SysDev &S, int si, int sj,
@@ -266,20 +285,7 @@ k_rows_count(const __grid_constant__ TraverseArgs a) {
     A.c[2] = hc.z;
     A.sys = hc.w;
     const SysDev &S = a.sys[A.sys];
-    A.p32 = a.pos32[A.si];
-    A.H.lo_rc = A.H.hi_rc = A.H.band = 0.f;
-    if (FP32) {
-        const double ext = (double)S.n[0] *
-                           fmax(fabs(S.bin[0][0]), fmax(fabs(S.bin[0][1]), fabs(S.bin[0][2])));
-        const double band =
-            guard_band(2.0 * ((double)a.amax[A.sys] + ext) + S.off_max + ext, S.cutoff);
-        A.H.lo_rc = __double2float_rd(S.cutoff_sq - band);
-        A.H.hi_rc = __double2float_ru(S.cutoff_sq + band);
-        A.H.band = __double2float_ru(band);
-    }
-    A.H.cutoff_sq = S.cutoff_sq;
-    A.H.ncut = S.ncutoffs;
-    A.H.pt_base = S.pt_base;
+    row_thresholds<FP32>(a, S, A);
     const int rows = on ? (2 * S.nscan[1] + 1) * (2 * S.nscan[2] + 1) : 0;
     RowList<WIDE> L;
     L.q = make_uint4(0u, 0u, 0u, 0u);

@@ -239,13 +239,14 @@ __device__ __forceinline__ void atom_lj(const TraverseArgs &a, int64_t si) {
         H.ncut = S.ncutoffs;
         H.pt_base = S.pt_base;
         const float wi = a.pos32[si].w;
-        const VisitDev *vt = a.visit + S.visit_base;
         const int nv = S.nvisit;
         for (int v = 0; v < nv; v++) {
-            const VisitDev &e = vt[v];
-            const int32_t d[3] = {e.d[0], e.d[1], e.d[2]};
-            int32_t cj[3], m[3];
+            int32_t d[3], cj[3], m[3];
+            float unused[3];
+            visit_at(a, S, v, d, unused);
             if (!visit_cell(S, cc, d, cj, m)) continue;
+            double off[3];
+            visit_vector(a, S, v, off);
             const int2 sl = cell_lookup(a, S, sys, cj[0], cj[1], cj[2]);
             if (checked_fail(sl.x < 0 || sl.y < sl.x || (long long)sl.y > a.natoms, a.err))
                 continue;
@@ -253,13 +254,13 @@ __device__ __forceinline__ void atom_lj(const TraverseArgs &a, int64_t si) {
             for (int32_t sj = sl.x; sj < sl.y; sj++) {
                 if (sj == self) continue;
                 const double4 pj = a.pos64[sj];
-                const double dx = dadd(dsub(pj.x, pi.x), e.off[0]);
-                const double dy = dadd(dsub(pj.y, pi.y), e.off[1]);
-                const double dz = dadd(dsub(pj.z, pi.z), e.off[2]);
+                const double dx = dadd(dsub(pj.x, pi.x), off[0]);
+                const double dy = dadd(dsub(pj.y, pi.y), off[1]);
+                const double dz = dadd(dsub(pj.z, pi.z), off[2]);
                 const double r2 = dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz));
                 if (!(r2 < H.cutoff_sq)) continue;
                 if (KIND != kCutScalar &&
-                    !exact_inside<KIND>(H, a, pi, pj, e.off, wi,
+                    !exact_inside<KIND>(H, a, pi, pj, off, wi,
                                         KIND == kCutPerType ? a.pos32[sj].w : 0.f))
                     continue;
                 lj_pair(a, dx, dy, dz, r2, f);

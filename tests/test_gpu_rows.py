@@ -98,3 +98,27 @@ def test_rows_of_a_range(oracle, rows):
     got = neighbour_list_rows("ijdDS", torch.from_numpy(pos).cuda(), cell, pbc, 2.1, rows)
     torch.cuda.synchronize()
     assert_same_lists(tuple(g.cpu().numpy() for g in got), tuple(w[keep] for w in want), "ijdDS")
+
+
+@pytest.mark.parametrize("n,edge,cutoff", [(1, 1.0, 52.0), (2, 1.3, 5.0), (700, 9.0, 2.5)])
+def test_forces_then_the_list(oracle, n, edge, cutoff):
+    """The force pass walks without a visit table (more visits than a table
+    holds) and with one; a list built right after it is the oracle's."""
+    import matscipy_neighbours as m
+    rng = np.random.default_rng(n)
+    cell = edge * np.array([[1.0, 0.0, 0.0], [0.1, 1.0, 0.0], [0.0, -0.2, 1.0]])
+    g = int(np.ceil(n ** (1.0 / 3.0)))
+    site = np.stack(np.meshgrid(*[np.arange(g)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n]
+    pos = (site + 0.2 * rng.uniform(size=(n, 3))) / g @ cell
+    i, D = oracle.oracle_neighbour_list("iD", cell, pos, cutoff, np.array([True] * 3))
+    r2 = (D * D).sum(axis=1)
+    s6 = (0.8 / r2) ** 3   # sigma^2 = 0.8
+    f = np.zeros((n, 3))
+    np.add.at(f, i, (-24.0 * s6 * (2.0 * s6 - 1.0) / r2)[:, None] * D)
+    scale = np.abs(24.0 * s6 * (2.0 * s6 + 1.0) / np.sqrt(r2)).sum()
+    e, got = m.lennard_jones(pos, cutoff, cell=cell, pbc=[True] * 3, sigma=np.sqrt(0.8))
+    assert np.abs(got - f).max() <= 1e-12 * scale
+    assert abs(e - 2.0 * np.sum(s6 * s6 - s6)) <= 1e-12 * np.sum(2.0 * (s6 * s6 + s6))
+    want = oracle.oracle_neighbour_list("ijS", cell, pos, cutoff, np.array([True] * 3))
+    assert_same_lists(m.neighbour_list("ijS", positions=pos, cell=cell, pbc=[True] * 3,
+                                       cutoff=cutoff), want, "ijS")
