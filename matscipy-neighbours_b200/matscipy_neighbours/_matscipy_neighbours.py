@@ -254,6 +254,12 @@ def quantity_flags(quantities):
     return flags
 
 
+def _data(a):
+    """Address of a numpy array's data (what ``a.ctypes.data`` gives, without
+    building a ctypes object)."""
+    return a.__array_interface__["data"][0]
+
+
 def _ptr(a):
     return None if a is None else ctypes.c_void_p(a.ctypes.data)
 
@@ -263,10 +269,10 @@ def make_request(flags, origin, cell, inv, pbc, nat, pos_ptr, on_device, cutoff,
                  aux_on_device=False):
     r = Request()
     r.quantities = flags
-    r.cell_origin = origin.ctypes.data
-    r.cell = cell.ctypes.data
-    r.inv_cell = inv.ctypes.data
-    r.pbc = pbc.ctypes.data
+    r.cell_origin = _data(origin)
+    r.cell = _data(cell)
+    r.inv_cell = _data(inv)
+    r.pbc = _data(pbc)
     r.nat = int(nat)
     r.positions = pos_ptr
     r.positions_on_device = 1 if on_device else 0
@@ -476,32 +482,21 @@ _NO_CONTEXT = _NoContext()
 
 
 def _device_outputs(torch, quantities, n, dev):
-    """The requested outputs as views of one device allocation (each starting
-    on a 256-byte boundary): one allocator call instead of one per quantity.
-    The views keep the allocation alive together."""
-    chars = [ch for ch in "ijDdS" if ch in quantities]
-    offs, total = {}, 0
-    for ch in chars:
-        extra, dt = _SHAPES[ch]
-        offs[ch] = total
-        total += (n * (3 if extra else 1) * np.dtype(dt).itemsize + 255) & ~255
-    raw = torch.empty(max(total, 1), dtype=torch.uint8, device=dev)
+    """One device tensor per requested quantity."""
     bufs = {}
-    for ch in chars:
-        extra, dt = _SHAPES[ch]
-        tdt = torch.int32 if dt == np.int32 else torch.float64
-        nbytes = n * (3 if extra else 1) * np.dtype(dt).itemsize
-        bufs[ch] = raw[offs[ch]:offs[ch] + nbytes].view(tdt).view((n,) + extra)
+    for ch in "ijDdS":
+        if ch in quantities:
+            extra, dt = _SHAPES[ch]
+            bufs[ch] = torch.empty((n,) + extra, device=dev,
+                                   dtype=torch.int32 if dt == np.int32 else torch.float64)
     return bufs
 
 
-def neighbour_list_dlpack(quantities, cell_origin, cell, inv_cell, pbc, host_pos,
-                          cutoffs, types=None, backend=0, py_in=None, device_id=-1):
-    """DLPack entry of the reference's extension (bind_py_dlpack.cc:231): a
-    tuple of "dltensor" capsules, one per quantity character.  backend 0
-    returns host capsules (the pairs are still computed on the GPU), backend 1
-    device capsules; `py_in` (anything with __dlpack__) supplies device
-    positions in place of `host_pos`."""
+def neighbour_list_tensors(quantities, cell_origin, cell, inv_cell, pbc, host_pos,
+                           cutoffs, types=None, backend=1, py_in=None, device_id=-1):
+    """``neighbour_list_dlpack`` with its results as arrays: host arrays for
+    backend 0 and host positions, else torch tensors on the device, one per
+    quantity character."""
     origin, cell, inv, pbc8, ty = _parse(quantities, cell_origin, cell, inv_cell, pbc,
                                          host_pos, cutoffs, types)
     hpos = _fromany(host_pos, np.float64, 2, 2)
@@ -516,17 +511,28 @@ def neighbour_list_dlpack(quantities, cell_origin, cell, inv_cell, pbc, host_pos
     if backend == 0 and not device_in:
         bufs = run_host(quantities, origin, cell, inv, pbc8, hpos, rc, per_atom,
                         per_type_sq, ncut, ty, flags, max(device_id, 0))
-        return tuple(a.__dlpack__() for a in _ordered(quantities, bufs))
+        return _ordered(quantities, bufs)
     dev_id = pos_t.device.index if device_in else max(device_id, 0)
     bufs = run_device(quantities, origin, cell, inv, pbc8, pos_t, hpos, rc, per_atom,
                       per_type_sq, ncut, ty, flags, dev_id)
     out = []
     seen = set()
     for ch in quantities:
-        t = bufs[ch]
-        out.append((t.clone() if ch in seen else t).__dlpack__())
+        out.append(bufs[ch].clone() if ch in seen else bufs[ch])
         seen.add(ch)
-    return tuple(out)
+    return out
+
+
+def neighbour_list_dlpack(quantities, cell_origin, cell, inv_cell, pbc, host_pos,
+                          cutoffs, types=None, backend=0, py_in=None, device_id=-1):
+    """DLPack entry of the reference's extension (bind_py_dlpack.cc:231): a
+    tuple of "dltensor" capsules, one per quantity character.  backend 0
+    returns host capsules (the pairs are still computed on the GPU), backend 1
+    device capsules; `py_in` (anything with __dlpack__) supplies device
+    positions in place of `host_pos`."""
+    return tuple(a.__dlpack__() for a in neighbour_list_tensors(
+        quantities, cell_origin, cell, inv_cell, pbc, host_pos, cutoffs, types, backend,
+        py_in, device_id))
 
 
 def coordination(cell_origin, cell, inv_cell, pbc, positions, cutoffs, types=None,
@@ -566,8 +572,19 @@ def neighbour_matrix_dlpack(cell_origin, cell, inv_cell, pbc, host_pos, cutoffs,
                             device_id=-1):
     """Dense (n x K) neighbour matrix (bind_py_dlpack.cc:500-658
     neighbour_matrix_dlpack): returns (idx, dist, count) capsules and the
-    overflow flag.  Rows hold each atom's neighbours in the reference's row
-    order, filled straight from the fill pass (no pair list in between)."""
+    overflow flag."""
+    outs, overflow = neighbour_matrix_tensors(cell_origin, cell, inv_cell, pbc, host_pos,
+                                              cutoffs, max_neighbours, types, backend,
+                                              py_in, device_id)
+    return tuple(t.__dlpack__() for t in outs) + (overflow,)
+
+
+def neighbour_matrix_tensors(cell_origin, cell, inv_cell, pbc, host_pos, cutoffs,
+                             max_neighbours, types=None, backend=1, py_in=None,
+                             device_id=-1):
+    """((idx, dist, count), overflow) as arrays.  Rows hold each atom's
+    neighbours in the reference's row order, filled straight from the fill pass
+    (no pair list in between)."""
     torch = _torch()
     origin, cell, inv, pbc8, ty = _parse("", cell_origin, cell, inv_cell, pbc,
                                          host_pos, cutoffs, types)
@@ -592,12 +609,14 @@ def neighbour_matrix_dlpack(cell_origin, cell, inv_cell, pbc, host_pos, cutoffs,
                        per_type_sq, ncut, ty, dev_id)
     npairs = ctypes.c_int64()
     overflow = ctypes.c_int(0)
-    with torch.cuda.device(dev):
+    ctx = torch.cuda.device(dev) if torch.cuda.current_device() != dev_id else _NO_CONTEXT
+    with ctx:
         check(lib.nbl_count(plan, ctypes.byref(req), ctypes.c_void_p(stream.cuda_stream),
                             ctypes.byref(npairs)))
-        idx = torch.zeros((nat, K), dtype=torch.int32, device=dev)
-        dist = torch.zeros((nat, K, 3), dtype=torch.float64, device=dev)
-        count = torch.zeros((nat,), dtype=torch.int32, device=dev)
+        # (the fill writes every slot, the unused ones with zeros)
+        idx = torch.empty((nat, K), dtype=torch.int32, device=dev)
+        dist = torch.empty((nat, K, 3), dtype=torch.float64, device=dev)
+        count = torch.empty((nat,), dtype=torch.int32, device=dev)
         if nat:
             check(lib.nbl_fill_matrix(plan, K, ctypes.c_void_p(idx.data_ptr()),
                                       ctypes.c_void_p(dist.data_ptr()),
@@ -607,7 +626,7 @@ def neighbour_matrix_dlpack(cell_origin, cell, inv_cell, pbc, host_pos, cutoffs,
     outs = (idx, dist, count)
     if backend == 0 and not device_in:
         outs = tuple(t.cpu().numpy() for t in outs)
-    return tuple(t.__dlpack__() for t in outs) + (bool(overflow.value),)
+    return outs, bool(overflow.value)
 
 
 # ---------------------------------------------------------------------------

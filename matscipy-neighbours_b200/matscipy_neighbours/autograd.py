@@ -45,7 +45,8 @@ def _function():
             pos = positions.detach().to(torch.float64).contiguous()
             cell_np = cell.detach().cpu().numpy().astype(np.float64)
             nat = pos.shape[0]
-            co, ce, inv, pb, nums = _host_metadata(cell_np, pbc, numbers, cell_origin, nat)
+            co, ce, inv, pb, nums = _host_metadata(cell_np, pbc, numbers, cell_origin, nat,
+                                                   cutoff=cutoff)
             rc, nums = _resolve_cutoff(cutoff, nums)
             rc, per_atom, per_type_sq, ncut = _ext.resolve_cutoff(rc, nat)
             pbc8 = np.ascontiguousarray(pb.astype(np.uint8))
@@ -65,12 +66,16 @@ def _function():
                 D = torch.empty((P, 3), dtype=torch.float64, device=dev)
                 d = torch.empty(P, dtype=torch.float64, device=dev)
                 S = torch.empty((P, 3), dtype=torch.int32, device=dev)
-                off = torch.empty(nat + 1, dtype=torch.int64, device=dev)
-                _ext.check(_ext.lib.nbl_row_offsets(plan, ctypes.c_void_p(off.data_ptr()), sp))
+                off = None  # (the default backward reads no row offsets)
+                if deterministic:
+                    off = torch.empty(nat + 1, dtype=torch.int64, device=dev)
+                    _ext.check(_ext.lib.nbl_row_offsets(plan, ctypes.c_void_p(off.data_ptr()),
+                                                        sp))
                 if P:
                     o = _ext._outputs_struct({"i": i, "j": j, "D": D, "d": d, "S": S},
                                              lambda t: t.data_ptr())
                     _ext.check(_ext.lib.nbl_fill(plan, ctypes.byref(o), sp))
+            ctx.set_materialize_grads(False)  # no zero gradients for i, j, S
             ctx.save_for_backward(i, j, S, D, d, off)
             ctx.pbc8 = pbc8
             ctx.nat = nat
@@ -95,7 +100,7 @@ def _function():
             a.distvec, a.absdist = D.data_ptr(), d.data_ptr()
             a.grad_distvec = gD.data_ptr() if gD is not None else None
             a.grad_absdist = gd.data_ptr() if gd is not None else None
-            a.row_offsets = off.data_ptr()
+            a.row_offsets = off.data_ptr() if off is not None else None
             a.pbc = ctx.pbc8.ctypes.data
             a.grad_positions = grad_pos.data_ptr()
             a.grad_cell = grad_cell.data_ptr()

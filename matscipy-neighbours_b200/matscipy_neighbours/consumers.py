@@ -43,7 +43,7 @@ def lennard_jones(positions, cutoff, *, cell, pbc=True, epsilon=1.0, sigma=1.0,
     nat = int(pos_t.shape[0])
     if not isinstance(cutoff, (int, float)):
         raise TypeError("lennard_jones takes one scalar cutoff")
-    co, ce, inv, pb, _ = _host_metadata(cell, pbc, None, cell_origin, nat)
+    co, ce, inv, pb, _ = _host_metadata(cell, pbc, None, cell_origin, nat, cutoff=float(cutoff))
     origin, ce, inv, pbc8 = _ext.coerce_geometry(co, ce, inv, pb)
     forces = torch.empty((nat, 3), dtype=torch.float64, device=dev)
     energy = torch.empty((), dtype=torch.float64, device=dev)

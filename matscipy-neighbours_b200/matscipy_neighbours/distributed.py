@@ -193,7 +193,8 @@ def neighbour_list_rows(quantities, positions, cell, pbc, cutoff, atom_range, *,
         raise ValueError(f"atom range [{lo}, {hi}) outside [0, {nat})")
     if cell is None:
         raise ValueError("cell must be given for device-resident positions.")
-    co, ce, inv, pb, nums = _host_metadata(cell, pbc, numbers, cell_origin, nat)
+    co, ce, inv, pb, nums = _host_metadata(cell, pbc, numbers, cell_origin, nat,
+                                           cutoff=cutoff)
     cut, nums = _resolve_cutoff(cutoff, nums)
     origin, ce, inv, pbc8 = _ext.coerce_geometry(co, ce, inv, pb)
     rc, per_atom, per_type_sq, ncut = _ext.resolve_cutoff(cut, nat)

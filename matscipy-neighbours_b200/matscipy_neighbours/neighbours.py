@@ -115,10 +115,15 @@ def _consume(wrappers, array_namespace, use_gpu):
     return [array_namespace.from_dlpack(w) for w in wrappers]
 
 
-def _host_metadata(cell, pbc, numbers, cell_origin, nat, *, positions=None):
+def _is_torch(namespace):
+    return getattr(namespace, "__name__", None) == "torch"
+
+
+def _host_metadata(cell, pbc, numbers, cell_origin, nat, *, positions=None, cutoff=None):
     """Normalise the host-side geometry (``neighbours.py:145-164``): cell
     shrink-wrapped around host positions when None, origin 0, pbc False,
-    numbers 1, inv_cell = inv(cell.T)."""
+    numbers 1 (left out for a float ``cutoff``, which reads none: a million
+    of them cost 150 us), inv_cell = inv(cell.T)."""
     if cell is None:
         r = np.asarray(positions, dtype=float)
         rmin, rmax = r.min(axis=0), r.max(axis=0)
@@ -128,12 +133,13 @@ def _host_metadata(cell, pbc, numbers, cell_origin, nat, *, positions=None):
         cell_origin = np.zeros(3)
     if pbc is None:
         pbc = np.zeros(3, dtype=bool)
-    if numbers is None:
+    if numbers is None and not isinstance(cutoff, float):
         numbers = np.ones(nat, dtype=np.int32)
     cell = np.ascontiguousarray(np.asarray(cell, dtype=float))
     cell_origin = np.ascontiguousarray(np.asarray(cell_origin, dtype=float))
     pbc = np.ascontiguousarray(np.broadcast_to(pbc, (3,)), dtype=bool)
-    numbers = np.ascontiguousarray(np.asarray(numbers), dtype=np.int32)
+    if numbers is not None:
+        numbers = np.ascontiguousarray(np.asarray(numbers), dtype=np.int32)
     inv_cell = np.ascontiguousarray(np.linalg.inv(cell.T))
     return cell_origin, cell, inv_cell, pbc, numbers
 
@@ -202,7 +208,8 @@ def neighbour_list(quantities, atoms=None, cutoff=None, *, positions=None,
     if not use_gpu and array_namespace is None:
         positions = np.ascontiguousarray(positions, dtype=float)
         co, ce, inv, pb, nums = _host_metadata(cell, pbc, numbers, cell_origin,
-                                               len(positions), positions=positions)
+                                               len(positions), positions=positions,
+                                               cutoff=cutoff)
         rc, nums = _resolve_cutoff(cutoff, nums)
         return _ext.neighbour_list(quantities, co, ce, inv, pb, positions, rc, nums)
 
@@ -215,8 +222,12 @@ def neighbour_list(quantities, atoms=None, cutoff=None, *, positions=None,
             device_id = 0
     co, ce, inv, pb, nums = _host_metadata(
         cell, pbc, numbers, cell_origin, nat,
-        positions=None if on_device else host_pos)
+        positions=None if on_device else host_pos, cutoff=cutoff)
     rc, nums = _resolve_cutoff(cutoff, nums)
+    if use_gpu and _is_torch(array_namespace):  # the engine's own tensors, no capsules
+        arrays = _ext.neighbour_list_tensors(quantities, co, ce, inv, pb, host_pos, rc,
+                                             nums, 1, py_in, device_id)
+        return arrays[0] if len(quantities) == 1 else tuple(arrays)
     capsules = _ext.neighbour_list_dlpack(quantities, co, ce, inv, pb, host_pos, rc,
                                           nums, 1 if use_gpu else 0, py_in, device_id)
     if use_gpu:
@@ -252,21 +263,23 @@ def neighbour_matrix(atoms=None, cutoff=None, max_neighbours=None, *,
             device_id = 0
     co, ce, inv, pb, nums = _host_metadata(
         cell, pbc, numbers, cell_origin, nat,
-        positions=None if on_device else host_pos)
+        positions=None if on_device else host_pos, cutoff=cutoff)
     rc, nums = _resolve_cutoff(cutoff, nums)
-    idx_cap, dist_cap, count_cap, overflow = _ext.neighbour_matrix_dlpack(
+    arrays, overflow = _ext.neighbour_matrix_tensors(
         co, ce, inv, pb, host_pos, rc, int(max_neighbours), nums,
         1 if use_gpu else 0, py_in, device_id)
     if overflow:
         raise ValueError(
             f"max_neighbours={max_neighbours} is too small: some atom has more "
             "neighbours than that. Retry with a larger max_neighbours.")
+    if use_gpu and _is_torch(array_namespace):
+        return tuple(arrays)
     if use_gpu:
         out_id = _dlpack_device(positions)[1] if on_device else device_id
         out_dev = (_ext._device_type, out_id)
     else:
         out_dev = (_DLPACK_CPU, 0)
-    wrappers = [DLPackTensor(c, out_dev) for c in (idx_cap, dist_cap, count_cap)]
+    wrappers = [DLPackTensor(t.__dlpack__(), out_dev) for t in arrays]
     return tuple(_consume(wrappers, array_namespace, use_gpu))
 
 
