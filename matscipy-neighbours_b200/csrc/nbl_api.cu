@@ -275,7 +275,7 @@ static ListPlan plan_lists(const Plan &p, const Batch &b) {
     const int64_t more = std::max<int64_t>(
         std::max<int64_t>(at / 4, known ? p.list_hint + p.list_hint / 4 : 0), int64_t(1) << 16);
     lp.total = at + more;
-    lp.row_cap = known && b.natoms > kMarkAtoms ? lp.total * 4 / kRowChunk + 16 : 0;
+    lp.row_cap = known && b.natoms > kMarkAtoms ? lp.total * 4 / kRowMark + 16 : 0;
     return lp;
 }
 int64_t ListPlan::cap(double m) const {

@@ -136,7 +136,7 @@ struct TraverseArgs {
     // (list_wide) two-word entries, of which those from list_chunks on are
     // handed out in chunks (mask_cursor); the sorted
     // atoms' home cells and systems, the sorted index of each atom, and the
-    // row of every kRowChunk-th output slot.
+    // row of every kRowMark-th output slot.
     uint4 *list;
     long long list_chunks, list_cap;
     int list_wide, list_shift;
@@ -147,7 +147,7 @@ struct TraverseArgs {
 };
 
 constexpr int kListChunk = 16;   // groups per chained chunk, the link included
-constexpr int kRowChunk = 256;   // output slots a fill warp takes at a time
+constexpr int kRowMark = 128;    // output slots between row marks
 
 // Launch shape of one pair pass: warps per CTA (2, 4 or 8, i.e. 64, 128 or
 // 256 threads), candidates staged per warp in the count (cand 0: 384 FP32 /

@@ -11,7 +11,7 @@
 // Neighbouring threads hold atoms of the same or adjacent cells, so a warp's
 // candidate loads are broadcasts.
 //
-// Fill (k_rows_fill).  A warp takes 256 consecutive output slots, finds the
+// Fill (k_rows_fill).  A warp takes 64 to 512 consecutive output slots, finds the
 // rows they belong to, and makes 32 consecutive slots a round: list entry, j's
 // record, the exact FP64 D and d, S.  Every store instruction covers whole
 // aligned lines of an output array, whatever the rows' lengths.
@@ -22,9 +22,9 @@
 // every row in each of five arrays.  Measured, count + fill: 200,000 atoms of a
 // slab with per-type cutoffs 84 + 25 us (187 + 120 one thread per atom writing
 // its own row), a gas of two neighbours per atom 62 + 23 (73 + 97); the fill
-// alone 653 us for the 88 M pairs of a million-atom metal (1,051 from hit words,
-// a warp per cell), bound by L1 wavefronts (71 %) and issue, and 5.4 TB/s of
-// output.
+// alone 612 us for the 46 M pairs of a million-atom metal (1,051 from hit words,
+// a warp per cell), 3.9 TB/s of output, bound by L1 wavefronts (75 %: position
+// gathers, staging) and the loads' latency.
 //
 // Which count: this one where the occupied cells hold fewer than kSparseAtoms
 // atoms on average, and with plain FP64 tests; k_count_list (nbl_trav_list.cu)
@@ -339,14 +339,14 @@ k_rows_count(const __grid_constant__ TraverseArgs a) {
     }
 }
 
-// Row of every kRowChunk-th output slot.
+// Row of every kRowMark-th output slot.
 __global__ void __launch_bounds__(256)
 k_row_marks(const int64_t *__restrict__ off, long long n, int32_t *__restrict__ row_of,
             long long row_cap) {
     const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
     if (i >= n) return;
     const long long e = off[i + 1];
-    for (long long c = (off[i] + kRowChunk - 1) / kRowChunk; c * kRowChunk < e && c < row_cap; c++)
+    for (long long c = (off[i] + kRowMark - 1) / kRowMark; c * kRowMark < e && c < row_cap; c++)
         row_of[c] = (int32_t)i;
 }
 
@@ -366,6 +366,9 @@ __device__ __forceinline__ long long find_row(const int64_t *off, long long n, l
 }
 
 constexpr int kFillWarps = 8;
+// CTAs per SM (48 registers a thread, no spills).  The million-atom metal's fill at
+// 3 / 4 / 5 / 6: 755 / 650 / 612 / 703 us; six of them spill and shrink the L1.
+constexpr int kFillBlocks = 5;
 
 struct __align__(16) RowWarp {
     double d[96];          // one round's distance vectors
@@ -431,32 +434,45 @@ __device__ __noinline__ void far_shift(const TraverseArgs &a, const SysDev &S, c
 }
 
 template <bool ALL5, bool WIDE>
-__global__ void __launch_bounds__(kFillWarps * 32, 4)
+__global__ void __launch_bounds__(kFillWarps * 32, kFillBlocks)
 k_rows_fill(const __grid_constant__ TraverseArgs a) {
     __shared__ RowWarp smem[kFillWarps];
+    __shared__ volatile long long last_chunk[kFillWarps][2];  // (spares registers)
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     RowWarp &sm = smem[warp];
     const long long total = a.offsets[a.natoms];
     const long long P = min(total, (long long)a.capacity);
     if (total > a.capacity && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(a.err, kErrCapacity);
-    const long long nchunks = (P + kRowChunk - 1) / kRowChunk;
-    const long long step = (long long)gridDim.x * kFillWarps;
-    for (long long ch = (long long)blockIdx.x * kFillWarps + warp; ch < nchunks; ch += step) {
-        const long long B0 = ch * kRowChunk;
-        const int E = (int)min((long long)kRowChunk, P - B0);  // slots of the chunk
-        long long row = ch < a.row_cap ? (long long)a.row_of[ch]
-                                       : find_row(a.offsets, a.natoms, B0, lane);
+    // Slots a warp takes at a time: a power of two from 64 to 512 that gives a warp
+    // about four chunks.  (At 128 / 256 / 512 the fill took 8.6 / 13 / 22 us for 65,000
+    // pairs, 19 / 24 / 39 for 400,000, 71 / 72 / 80 for 5.4 M, 660 / 610 / 610 for
+    // 46 M, 1,189 / 1,144 / 1,093 for the batch of 4,096 systems.)
+    const int step = (int)gridDim.x * kFillWarps;
+    int bits = 6;
+    while (bits < 9 && (P >> bits) > 4ll * step) bits++;
+    const int nchunks = (int)((P + (1 << bits) - 1) >> bits);
+    last_chunk[warp][0] = P;
+    last_chunk[warp][1] = nchunks;
+    __syncwarp();
+    for (int ch = (int)blockIdx.x * kFillWarps + warp; ch < (int)last_chunk[warp][1]; ch += step) {
+        const long long B0 = (long long)ch << bits;
+        const int E = (int)min(1ll << bits, last_chunk[warp][0] - B0);  // slots of the chunk
+        int row;
+        if ((B0 & (kRowMark - 1)) == 0 && B0 / kRowMark < a.row_cap)
+            row = a.row_of[B0 / kRowMark];
+        else
+            row = (int)find_row(a.offsets, a.natoms, B0, lane);
         int pos = 0;
         while (pos < E && row < a.natoms) {
             // --- the next 32 rows: the non-empty ones, compacted ---------------------
-            const long long r = row + lane;
+            const int r = row + lane;
             long long o0 = 0, o1 = 0;
             if (r < a.natoms) {
                 o0 = a.offsets[r];
                 o1 = a.offsets[r + 1];
             }
-            const long long wend = __shfl_sync(full, o1, (int)min(31ll, a.natoms - 1 - row));
+            const long long wend = __shfl_sync(full, o1, min(31, (int)a.natoms - 1 - row));
             const bool take = o1 > o0 && o0 < B0 + E;
             const unsigned mask = __ballot_sync(full, take);
             const int nrow = __popc(mask);
@@ -660,7 +676,7 @@ cudaError_t launch_row_marks(const TraverseArgs &a, cudaStream_t st) {
 cudaError_t launch_fill_rows(const TraverseArgs &a, int num_sms, cudaStream_t st) {
     if (a.natoms <= 0) return cudaSuccess;
     const TravKernel k = a.list_wide ? fill_kernel<true>(a) : fill_kernel<false>(a);
-    k<<<(unsigned)(num_sms * 4), kFillWarps * 32, 0, st>>>(a);
+    k<<<(unsigned)(num_sms * kFillBlocks), kFillWarps * 32, 0, st>>>(a);
     count_launch();
     return cudaGetLastError();
 }
