@@ -437,6 +437,19 @@ NBL_API nbl_status nbl_triplet_list(int64_t nfirst, const int32_t *first_i,
                                     int32_t *ik, int64_t capacity, int64_t *ntriplets,
                                     void *stream);
 
+/* The same in two calls, for callers that allocate in between:
+   nbl_triplet_count fills row_offsets (device, nfirst + 1 entries: each row's
+   first triplet, the total, and a word of its own) and sets *ntriplets
+   (synchronises `stream`); nbl_triplet_fill writes ij/ik from them
+   (asynchronous). */
+NBL_API nbl_status nbl_triplet_count(int64_t nfirst, const int32_t *first_i,
+                                     const double *absdist, double cutoff,
+                                     int64_t *row_offsets, int64_t *ntriplets, void *stream);
+NBL_API nbl_status nbl_triplet_fill(int64_t nfirst, const int32_t *first_i,
+                                    const double *absdist, double cutoff,
+                                    const int64_t *row_offsets, int32_t *ij, int32_t *ik,
+                                    void *stream);
+
 /* Allocation-free variant of nbl_count + nbl_fill, for callers that cannot
    allocate device memory at call time (an MD loop that forbids allocation
    after start-up, a host whose pool allocator has reserved the device

@@ -123,6 +123,10 @@ def _load():
                            P], ctypes.c_int),
         "nbl_triplet_list": ([ctypes.c_int64, P, P, ctypes.c_double, P, P, ctypes.c_int64,
                               ctypes.POINTER(ctypes.c_int64), P], ctypes.c_int),
+        "nbl_triplet_count": ([ctypes.c_int64, P, P, ctypes.c_double, P,
+                               ctypes.POINTER(ctypes.c_int64), P], ctypes.c_int),
+        "nbl_triplet_fill": ([ctypes.c_int64, P, P, ctypes.c_double, P, P, P, P],
+                             ctypes.c_int),
     }
     for name, (args, res) in sigs.items():
         fn = getattr(lib, name)
@@ -722,7 +726,8 @@ def triplet_list(first_i, absdist=None, cutoff=None):
 
 
 def _triplet_list_device(ft, absdist, cutoff):
-    """triplet_list on the GPU of `ft` (nbl_triplet_list): torch CUDA tensors."""
+    """triplet_list on the GPU of `ft` (nbl_triplet_count, nbl_triplet_fill): torch
+    CUDA tensors."""
     torch = _torch()
     if absdist is not None and cutoff is None:
         raise TypeError("triplet_list: distances given without a cutoff")
@@ -739,14 +744,16 @@ def _triplet_list_device(ft, absdist, cutoff):
     dp = ctypes.c_void_p(dt.data_ptr()) if dt is not None and dt.numel() else None
     c = float(cutoff) if cutoff is not None else 0.0
     n = ctypes.c_int64()
-    with torch.cuda.device(ft.device):
-        check(lib.nbl_triplet_list(int(ft.shape[0]), fp, dp, c, None, None, 0,
-                                   ctypes.byref(n), sp))
+    nf = int(ft.shape[0])
+    ctx = (torch.cuda.device(ft.device) if torch.cuda.current_device() != ft.device.index
+           else _NO_CONTEXT)
+    with ctx:
+        off = torch.empty(nf + 1, dtype=torch.int64, device=ft.device)
+        op = ctypes.c_void_p(off.data_ptr())
+        check(lib.nbl_triplet_count(nf, fp, dp, c, op, ctypes.byref(n), sp))
         ij = torch.empty(int(n.value), dtype=torch.int32, device=ft.device)
         ik = torch.empty(int(n.value), dtype=torch.int32, device=ft.device)
         if n.value:
-            check(lib.nbl_triplet_list(int(ft.shape[0]), fp, dp, c,
-                                       ctypes.c_void_p(ij.data_ptr()),
-                                       ctypes.c_void_p(ik.data_ptr()), int(n.value),
-                                       ctypes.byref(n), sp))
+            check(lib.nbl_triplet_fill(nf, fp, dp, c, op, ctypes.c_void_p(ij.data_ptr()),
+                                       ctypes.c_void_p(ik.data_ptr()), sp))
     return ij, ik
