@@ -52,11 +52,10 @@ struct __align__(16) ListWarp {
     int32_t bj[kSeg];           // candidate kk of the segment is sorted atom bj + kk
     int32_t pref[kSeg + 1];
 };
-constexpr int list_blocks(bool wide, bool cull) {
-    return wide || cull ? 4 : 5;  // CTAs per SM
-}
-static_assert(list_blocks(false, false) * (kListWarps * sizeof(ListWarp<false>) + 1024) <= 233472 &&
-                  list_blocks(true, true) * (kListWarps * sizeof(ListWarp<true>) + 1024) <= 233472,
+// CTAs per SM.  (Culling, 4,096 small systems: 1,557 us at 5, 1,615 at 4.)
+constexpr int list_blocks(bool wide) { return wide ? 4 : 5; }
+static_assert(list_blocks(false) * (kListWarps * sizeof(ListWarp<false>) + 1024) <= 233472 &&
+                  list_blocks(true) * (kListWarps * sizeof(ListWarp<true>) + 1024) <= 233472,
               "the CTAs fit the SM's shared memory");
 
 // Segment batch vb of the item's home cell: one lane per visited offset
@@ -310,7 +309,7 @@ __device__ __forceinline__ void list_pair(ListWarp<WIDE> &sm, const TraverseArgs
 }
 
 template <int KIND, bool WIDE, bool CULL>
-__global__ void __launch_bounds__(kListWarps * 32, list_blocks(WIDE, CULL))
+__global__ void __launch_bounds__(kListWarps * 32, list_blocks(WIDE))
 k_count_list(const __grid_constant__ TraverseArgs a) {
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     using E = Entry<WIDE>;
@@ -491,7 +490,7 @@ cudaError_t launch(int kind, const TraverseArgs &a, int num_sms, cudaStream_t st
                          : kind == kCutPerType ? k_count_list<kCutPerType, WIDE, CULL>
                                                : k_count_list<kCutScalar, WIDE, CULL>;
     const int64_t grid =
-        std::min<int64_t>((int64_t)num_sms * list_blocks(WIDE, CULL), (a.natoms + 3) / 4);
+        std::min<int64_t>((int64_t)num_sms * list_blocks(WIDE), (a.natoms + 3) / 4);
     return launch_kernel(k, sizeof(ListWarp<WIDE>) * kListWarps, kListWarps, a, (int)grid, st);
 }
 
