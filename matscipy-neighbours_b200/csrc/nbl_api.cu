@@ -545,14 +545,26 @@ static bool sparse_grid(const Plan &p, const Batch &b) {
     return (double)b.natoms < kSparseAtoms * cells;
 }
 
+// Whether the force pass takes one thread per atom (k_atoms_lj) instead of the
+// work items (k_count_list): for cutoffs by atom or type, and on sparse grids.
+// Measured (us, by items / by atoms): 200,001 atoms at 1 / 2.9 / 3.3 / 13 per cell
+// 214 / 64, 152 / 117, 145 / 121, 198 / 249; 20,001 atoms at 0.5 / 1.4 / 2.4 / 13
+// 31 / 25, 31 / 47, 25 / 53, 50 / 129; 7,483 at 11 24 / 101.
+static bool lj_by_atoms(const Batch &b) {
+    if (b.sys.empty() || b.sys[0].cutoff_kind != kCutScalar) return true;
+    double cells = 0.0;
+    for (int64_t n : b.ncells) cells += (double)n;
+    return (double)b.natoms < (b.natoms <= 65536 ? 1.0 : 4.0) * cells;
+}
+
 // Size the workspace for a batch and copy its inputs and host tables in.
 nbl_status upload_batch(Plan &p, const Batch &b, cudaStream_t st, CountUse use) {
     // the row passes, unless the one-launch count phase or the launch
-    // configuration asks for the warp passes or the thread-per-atom passes; a
-    // force pass walks as the sparse count does
+    // configuration asks for the warp passes or the thread-per-atom passes
     p.forces = use == kUseForces;
     p.rows = p.forces || (use == kUseLists && p.atom_threads == 0 && p.max_run == 0);
-    p.sparse = p.forces || (p.rows && (!b.fp32 || sparse_grid(p, b)));
+    p.sparse = p.rows && (!b.fp32 || sparse_grid(p, b));
+    if (p.forces) p.sparse = !b.fp32 || lj_by_atoms(b);
     p.cand_atom = candidates_per_atom(b);
     nbl_status s = layout_workspace(p, b);
     if (s != NBL_SUCCESS) return s;
@@ -1510,7 +1522,10 @@ nbl_status nbl_lj_forces(nbl_plan *plan, const nbl_request *req, double epsilon,
     ta.lj_eps4 = 4.0 * epsilon;
     ta.lj_eps24 = 24.0 * epsilon;
     ta.lj_sig2 = sigma * sigma;
-    NBL_CUDA(launch_lj_atoms(p.batch_kind, ta, cs), "force pass");
+    ta.ticket_ready = 1;  // k_init cleared the ticket
+    NBL_CUDA(p.sparse ? launch_lj_atoms(p.batch_kind, ta, cs)
+                      : launch_lj_list(p.cand_atom > kCullCand, ta, p.num_sms, cs),
+             "force pass");
     NBL_CUDA(launch_lj_energy(p.bufs.lj_part, b.natoms, p.bufs.lj_part + b.natoms, energy,
                               cs),
              "energy");

@@ -262,7 +262,9 @@ cudaError_t launch_count_list(int kind, bool cull, const TraverseArgs &a, int nu
                               cudaStream_t st);
 cudaError_t launch_row_marks(const TraverseArgs &a, cudaStream_t st);
 cudaError_t launch_fill_rows(const TraverseArgs &a, int num_sms, cudaStream_t st);
-// Lennard-Jones forces (TraverseArgs::lj_*) without a count, one thread per atom.
+// Lennard-Jones forces (TraverseArgs::lj_*) without a count: by work items (scalar
+// cutoffs), or one thread per atom.
+cudaError_t launch_lj_list(bool cull, const TraverseArgs &a, int num_sms, cudaStream_t st);
 cudaError_t launch_lj_atoms(int kind, const TraverseArgs &a, cudaStream_t st);
 int occupancy_fill_fp32(int kind, const TravShape &shape);
 int occupancy_fill_fp64(int kind, const TravShape &shape);

@@ -222,7 +222,9 @@ __device__ __forceinline__ void atom_row(const TraverseArgs &a, int64_t si) {
     }
 }
 
-// One sorted atom's Lennard-Jones force and energy share, over the same walk.
+// One sorted atom's Lennard-Jones force and energy share, over the same walk:
+// sparse grids (below the force pass's line by work items), other cutoff kinds
+// and plain FP64 tests.
 template <int KIND>
 __device__ __forceinline__ void atom_lj(const TraverseArgs &a, int64_t si) {
     const double4 pi = a.pos64[si];

@@ -122,3 +122,32 @@ def test_forces_then_the_list(oracle, n, edge, cutoff):
     want = oracle.oracle_neighbour_list("ijS", cell, pos, cutoff, np.array([True] * 3))
     assert_same_lists(m.neighbour_list("ijS", positions=pos, cell=cell, pbc=[True] * 3,
                                        cutoff=cutoff), want, "ijS")
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("n,edge,cutoff", [(33, 4.0, 1.9), (1000, 10.0, 2.5), (4097, 14.0, 2.5),
+                                           (900, 60.0, 2.5), (400, 6.2, 3.0)])
+def test_forces_by_items_and_by_atoms(oracle, n, edge, cutoff, precision):
+    """Force passes by work items (tiles of every size, many candidates) and by
+    atoms (sparse, plain FP64) against the pair list."""
+    import matscipy_neighbours as m
+    from matscipy_neighbours import _matscipy_neighbours as ext
+    rng = np.random.default_rng(n)
+    cell = edge * np.array([[1.0, 0.0, 0.0], [0.1, 1.0, 0.0], [0.0, -0.2, 1.0]])
+    g = int(np.ceil(n ** (1.0 / 3.0)))
+    site = np.stack(np.meshgrid(*[np.arange(g)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n]
+    pos = (site + 0.2 * rng.uniform(size=(n, 3))) / g @ cell
+    pbc = np.array([True, False, True])
+    i, D = oracle.oracle_neighbour_list("iD", cell, pos, cutoff, pbc)
+    r2 = (D * D).sum(axis=1)
+    s6 = (0.8 / r2) ** 3
+    f = np.zeros((n, 3))
+    np.add.at(f, i, (-24.0 * s6 * (2.0 * s6 - 1.0) / r2)[:, None] * D)
+    scale = np.abs(24.0 * s6 * (2.0 * s6 + 1.0) / np.sqrt(r2)).sum() + 1e-300
+    prev = ext.set_options(precision=precision)
+    try:
+        e, got = m.lennard_jones(pos, cutoff, cell=cell, pbc=pbc, sigma=np.sqrt(0.8))
+    finally:
+        ext.set_options(**prev)
+    assert np.abs(got - f).max() <= 1e-12 * scale
+    assert abs(e - 2.0 * np.sum(s6 * s6 - s6)) <= 1e-12 * (np.sum(2.0 * (s6 * s6 + s6)) + 1e-300)
