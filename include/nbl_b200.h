@@ -154,7 +154,11 @@ NBL_API nbl_status nbl_plan_set_launch(nbl_plan *plan, int count_ctas_per_sm, in
 
 /* The full launch configuration of the pair passes (what the batch
    autotuner chooses; a single call uses the defaults unless set here).  Every
-   value gives bit-identical output.  Zero fields mean the default.
+   value gives bit-identical output.  Zero fields mean the default.  By default
+   the pair passes go through neighbour lists (the row passes), which take
+   atoms_per_item from here and nothing else; the other shapes are the warp
+   passes', which thread_per_atom = -1 or a nonzero cells_per_item asks for, and
+   which a one-launch count phase uses.
      count_ctas_per_sm, fill_ctas_per_sm  grid of each pass (0: two waves of
                                           its resident CTAs), <= 64
      count_strided, fill_strided          work items by a fixed warp stride
@@ -173,11 +177,13 @@ NBL_API nbl_status nbl_plan_set_launch(nbl_plan *plan, int count_ctas_per_sm, in
                                           65,536, else 32
      cells_per_item                       home cells one work item may join
                                           along x when their atoms fit one
-                                          tile: 0 = chosen on the device from
-                                          the mean cell occupancy (sparse
-                                          grids join up to 8), 1 = one cell
-                                          per item, 2..8 = at most that many
-                                          (dense grid and FP32 filter only)
+                                          tile: 0 = the row passes (with
+                                          thread_per_atom = -1: chosen on the
+                                          device from the mean cell occupancy,
+                                          sparse grids join up to 8), 1 = one
+                                          cell per item, 2..8 = at most that
+                                          many (dense grid and FP32 filter
+                                          only)
      one_launch_atoms                     systems of up to this many atoms
                                           (one system, dense grid of at most
                                           16,384 cells) run the whole count
@@ -185,17 +191,17 @@ NBL_API nbl_status nbl_plan_set_launch(nbl_plan *plan, int count_ctas_per_sm, in
                                           128 atoms, else a thread-block
                                           cluster of up to 8 CTAs):
                                           0 = the default, -1 = never, 1..2048
-     thread_per_atom                      pair passes with one thread per atom
-                                          instead of one warp per work item:
-                                          0 = where the occupied cells hold
-                                          fewer than two atoms on average
-                                          (known after a first count of the
-                                          same sizes; before it, fewer atoms
-                                          than cells), -1 =
-                                          never, 1 = always (systems with a
-                                          visit table: at most 2^20 visited
-                                          offsets in all); the force sink
-                                          always uses work items
+     thread_per_atom                      0 = the row passes, whose count takes
+                                          one thread per atom where the
+                                          occupied cells hold fewer than four
+                                          atoms on average (known after a first
+                                          count of the same sizes; before it
+                                          empty cells count too), -1 = the warp
+                                          passes, 1 = one thread per atom in
+                                          both passes, without lists (systems
+                                          with a visit table: at most 2^20
+                                          visited offsets in all); the force
+                                          pass does not depend on it
    No reference counterpart (the reference has no tuner). */
 typedef struct nbl_launch_config {
     int count_ctas_per_sm;
@@ -377,7 +383,7 @@ NBL_API nbl_status nbl_backward(const nbl_backward_args *args, void *stream);
 
 /* Forces and energy of a truncated Lennard-Jones pair potential over the
    request's neighbour pairs, U = 4 eps ((sigma/r)^12 - (sigma/r)^6) for
-   r < cutoff, computed inside the fill pass: no pair is written.  forces
+   r < cutoff, computed inside one sweep: no pair is written.  forces
    (device, 3 * nat doubles, original atom order) receives F_i = -dU/dr_i
    summed over the pairs of row i; *energy (device, one double) receives
    sum over pairs of U / 2 per directed pair, i.e. each unordered pair once.
