@@ -300,7 +300,9 @@ static nbl_status layout_workspace(Plan &p, const Batch &b) {
     const int64_t hist = counted ? 0 : radix_hist_elems(std::max<int64_t>(N, 1));
     Layout L;
     Bufs &B = p.bufs;
-    size_t o_pos = b.pos_on_device ? 0 : L.add(sizeof(double) * 3 * N);
+    // small host positions travel with the host tables, in one upload
+    const bool pos_in_tab = !b.pos_on_device && N > 0 && N <= kTablePositions;
+    size_t o_pos = b.pos_on_device || pos_in_tab ? 0 : L.add(sizeof(double) * 3 * N);
     size_t o_pa = (b.per_atom && !b.aux_on_device) ? L.add(sizeof(double) * N) : 0;
     size_t o_ty = (b.types && !b.aux_on_device) ? L.add(sizeof(int32_t) * N) : 0;
     // the small host tables, contiguous (one upload)
@@ -308,6 +310,7 @@ static nbl_status layout_workspace(Plan &p, const Batch &b) {
     size_t o_sab = L.add(sizeof(int64_t) * nsys);
     size_t o_pt64 = L.add(sizeof(double) * std::max<size_t>(b.pt64.size(), 1));
     size_t o_pt32 = L.add(sizeof(float) * std::max<size_t>(b.pt64.size(), 1));
+    if (pos_in_tab) o_pos = L.add(sizeof(double) * 3 * N);
     const size_t tab_end = L.total;
     const int64_t nvis = visit_entries(b);
     size_t o_vis = nvis ? L.add(sizeof(VisitDev) * nvis) : 0;
@@ -363,6 +366,7 @@ static nbl_status layout_workspace(Plan &p, const Batch &b) {
     B.tab_pt64 = o_pt64 - o_sys;
     B.tab_pt32 = o_pt32 - o_sys;
     B.tab_bytes = tab_end - o_sys;
+    B.tab_pos = pos_in_tab ? o_pos - o_sys : 0;
     B.visit = nvis ? (VisitDev *)at(o_vis) : nullptr;
     B.sys_atom_base = (int64_t *)at(o_sab);
     B.pt64 = (double *)at(o_pt64);
@@ -577,9 +581,10 @@ nbl_status upload_batch(Plan &p, const Batch &b, cudaStream_t st, CountUse use) 
     p.batch_grid = b.grid;
     p.have_count = false;
     p.count_pending = false;
+    p.spare_ticket = false;
     p.lists_short = true;  // until a synchronised count says otherwise
 
-    if (!b.pos_on_device && N > 0)
+    if (!b.pos_on_device && N > 0 && B.tab_pos == 0)
         NBL_CUDA(cudaMemcpyAsync(B.pos, b.positions, sizeof(double) * 3 * N,
                                  cudaMemcpyHostToDevice, st), "copy positions");
     if (b.per_atom && !b.aux_on_device && N > 0)
@@ -626,6 +631,7 @@ nbl_status upload_batch(Plan &p, const Batch &b, cudaStream_t st, CountUse use) 
                 base += hs[s2].nvisit;
             }
         }
+        if (B.tab_pos != 0) std::memcpy(h + B.tab_pos, b.positions, sizeof(double) * 3 * N);
         int64_t *sab = reinterpret_cast<int64_t *>(h + B.tab_sab);
         for (int s2 = 0; s2 < nsys; s2++) sab[s2] = b.sys[s2].atom_base;
         if (!b.pt64.empty()) {
@@ -1014,6 +1020,7 @@ nbl_status run_count(Plan &p, const Batch &b, cudaStream_t st, bool sync) {
     } else {
         s = small ? enqueue_count_small(p, b, st) : enqueue_count(p, b, st);
         if (s != NBL_SUCCESS) return s;
+        p.spare_ticket = small;  // word 7, cleared and not used since
     }
     Bufs &B = p.bufs;
     const int64_t N = b.natoms;
@@ -1064,6 +1071,11 @@ nbl_status run_fill(Plan &p, const nbl_outputs &o, int64_t capacity, cudaStream_
         // rows without a list (none where a synchronised count said so)
         if (p.lists_short) NBL_CUDA(launch_fill_atoms(p.batch_kind, ta, st), "fill pass");
         return NBL_SUCCESS;
+    }
+    if (p.spare_ticket && ta.item_next != nullptr) {  // no reset for the first fill
+        ta.item_next = p.bufs.small + 7;
+        ta.ticket_ready = 1;
+        p.spare_ticket = false;
     }
     NBL_CUDA(launch_traverse(kModeFill, p.batch_fp32, p.batch_kind, ta, p.fill_grid, st,
                              p.fill_shape),

@@ -76,7 +76,7 @@ struct Bufs {
     // The small host tables (systems, their atom bases, per-type cutoffs in
     // FP64 and FP32) lie at these byte offsets from `sys`, one contiguous
     // block of tab_bytes, so that they go up in one copy.
-    size_t tab_sab = 0, tab_pt64 = 0, tab_pt32 = 0, tab_bytes = 0;
+    size_t tab_pos = 0, tab_sab = 0, tab_pt64 = 0, tab_pt32 = 0, tab_bytes = 0;
     uint32_t *mask_pool = nullptr;
     long long mask_cap = 0;
     long long *home_mask = nullptr;
@@ -106,6 +106,9 @@ constexpr int kAutoWaves = 2;
 // without, fill + marks: 1,048,576 atoms 657 against 699 us, 200,000 27 against
 // 27, 132,651 76 against 76, 1,000 16 against 13.
 constexpr int64_t kMarkAtoms = 131072;
+// Host positions of up to this many atoms are uploaded with the host tables: one
+// copy from pinned memory instead of that and one from pageable memory.
+constexpr int64_t kTablePositions = 2048;
 // Atoms per occupied cell below which the count takes one thread per atom
 // (k_rows_count against k_count_list: 84 / 214 us at 2.3, 674 / 490 at 10).
 constexpr double kSparseAtoms = 4.0;
@@ -171,6 +174,7 @@ struct Plan {
     double cand_atom = 0.0;   // atoms of the cells that an atom visits, on average
     bool forces = false;      // a force pass: no lists planned
     bool sparse = false;      // with one thread per atom in the count
+    bool spare_ticket = false;  // a cleared work-item ticket is left for one fill
     bool lists_short = true;  // some row may have no list (kErrNoList)
     int64_t list_natoms = -1, list_table = -1, list_hint = 0;
     double list_scale = 1.0;
