@@ -22,8 +22,8 @@
 // every row in each of five arrays.  Measured, count + fill: 200,000 atoms of a
 // slab with per-type cutoffs 84 + 25 us (187 + 120 one thread per atom writing
 // its own row), a gas of two neighbours per atom 62 + 23 (73 + 97); the fill
-// alone 612 us for the 46 M pairs of a million-atom metal (1,051 from hit words,
-// a warp per cell), 3.9 TB/s of output, bound by L1 wavefronts (75 %: position
+// alone 612 us for the 48 M pairs of a million-atom metal (1,051 from hit words,
+// a warp per cell), 4.0 TB/s of output, bound by L1 wavefronts (75 %: position
 // gathers, staging) and the loads' latency.
 //
 // Which count: this one where the occupied cells hold fewer than kSparseAtoms
@@ -447,7 +447,7 @@ k_rows_fill(const __grid_constant__ TraverseArgs a) {
     // Slots a warp takes at a time: a power of two from 64 to 512 that gives a warp
     // about four chunks.  (At 128 / 256 / 512 the fill took 8.6 / 13 / 22 us for 65,000
     // pairs, 19 / 24 / 39 for 400,000, 71 / 72 / 80 for 5.4 M, 660 / 610 / 610 for
-    // 46 M, 1,189 / 1,144 / 1,093 for the batch of 4,096 systems.)
+    // 48 M, 1,189 / 1,144 / 1,093 for the batch of 4,096 systems.)
     const int step = (int)gridDim.x * kFillWarps;
     int bits = 6;
     while (bits < 9 && (P >> bits) > 4ll * step) bits++;
@@ -577,9 +577,11 @@ k_rows_fill(const __grid_constant__ TraverseArgs a) {
 }
 
 // The neighbour matrix: a warp per row, ranks in rounds of 32, the slots past
-// the row's end set to zero.
+// the row's end set to zero (so nothing clears the matrix first).  Bound by its
+// writes, 28 bytes a slot: 131,072 rows of 64 slots 70 us, 3.3 TB/s (105 from hit
+// words, a warp per cell, after 89 of clearing); 74 at four CTAs per SM.
 template <bool WIDE>
-__global__ void __launch_bounds__(kFillWarps * 32, 4)
+__global__ void __launch_bounds__(kFillWarps * 32, kFillBlocks)
 k_rows_matrix(const __grid_constant__ TraverseArgs a) {
     __shared__ double sd[kFillWarps][96];
     const unsigned full = 0xffffffffu;
