@@ -247,8 +247,8 @@ static double list_entries(double m) { return 1.1 * m + 4.0 * std::sqrt(m) + 4.0
 // Sizes of the neighbour lists: every system's entries per atom follow its
 // density, scaled by what the last count of the same sizes found (surfaces,
 // cutoffs below the widest); a quarter on top, or what the last count took
-// and more, for chained chunks.
-static ListPlan plan_lists(const Plan &p, const Batch &b) {
+// and more, for chained chunks; at most about `most` entries.
+static ListPlan plan_lists(const Plan &p, const Batch &b, int64_t most) {
     ListPlan lp;
     const bool known =
         !p.forces && p.list_natoms == b.natoms && p.list_table == b.table_size;
@@ -267,13 +267,14 @@ static ListPlan plan_lists(const Plan &p, const Batch &b) {
     }
     lp.expect = mean;
     lp.scale = scale;
-    // at most 2^30 entries up front
-    lp.shrink = own > (double)(int64_t(1) << 30) ? (double)(int64_t(1) << 30) / own : 1.0;
+    lp.shrink = own > (double)most ? (double)most / own : 1.0;
     int64_t at = 0;
     for (size_t s = 0; s < b.sys.size(); s++) at += lp.cap(expected_row(b, s)) * b.sys[s].nat;
     lp.chunks = at;
-    const int64_t more = std::max<int64_t>(
-        std::max<int64_t>(at / 4, known ? p.list_hint + p.list_hint / 4 : 0), int64_t(1) << 16);
+    const int64_t more = std::min(
+        std::max<int64_t>(std::max<int64_t>(at / 4, known ? p.list_hint + p.list_hint / 4 : 0),
+                          int64_t(1) << 16),
+        most / 4);
     lp.total = at + more;
     lp.row_cap = known && b.natoms > kMarkAtoms ? lp.total * 4 / kRowMark + 16 : 0;
     return lp;
@@ -292,8 +293,9 @@ static bool counted_cells(const Batch &b) {
            b.table_size <= std::max<int64_t>(int64_t(1) << 20, 8 * b.natoms);
 }
 
-// Carve the per-call buffers out of the plan's workspace.
-static nbl_status layout_workspace(Plan &p, const Batch &b) {
+// Carve the per-call buffers out of the plan's workspace, with lists of at most
+// about `most_list` entries.
+static nbl_status layout_workspace(Plan &p, const Batch &b, int64_t most_list) {
     const int64_t N = b.natoms;
     const int64_t nsys = (int64_t)b.sys.size();
     const bool counted = counted_cells(b);
@@ -340,7 +342,7 @@ static nbl_status layout_workspace(Plan &p, const Batch &b) {
     size_t o_hmask =
         p.rows ? 0 : L.add(sizeof(long long) * std::max<int64_t>(N, 1) * kMaskBatches);
     size_t o_items = p.sparse ? 0 : L.add(sizeof(WorkItem) * std::max<int64_t>(N, 1));
-    const ListPlan lp = p.rows ? plan_lists(p, b) : ListPlan();
+    const ListPlan lp = p.rows ? plan_lists(p, b, most_list) : ListPlan();
     size_t o_list = L.add(sizeof(uint4) * lp.total);
     size_t o_hcell = p.rows ? L.add(sizeof(int4) * N) : 0;
     size_t o_inv = p.rows ? L.add(sizeof(int32_t) * N) : 0;
@@ -401,6 +403,17 @@ static nbl_status layout_workspace(Plan &p, const Batch &b) {
     B.list_plan = lp;
     B.lj_part = (double *)at(o_ljp);
     return NBL_SUCCESS;
+}
+
+// The same with lists for every expected pair or, where the device has no room for
+// them, few: rows without room are written by the thread-per-atom fill.
+static nbl_status layout_workspace(Plan &p, const Batch &b) {
+    constexpr int64_t kMost = int64_t(1) << 32, kFew = int64_t(1) << 26;
+    const nbl_status st = layout_workspace(p, b, kMost);
+    if (st != NBL_ERROR_OUT_OF_MEMORY || !p.rows || 4 * plan_lists(p, b, kMost).total <= kFew)
+        return st;
+    clear_error();
+    return layout_workspace(p, b, kFew);
 }
 
 // ---------------------------------------------------------------------------
