@@ -391,7 +391,10 @@ NBL_API nbl_status nbl_backward(const nbl_backward_args *args, void *stream);
    input errors.  The same pair set as nbl_count/nbl_fill, so the forces are
    those of the reference's pair list (lj_langevin_gpu.cu:59-74, the
    reference's example, with eps = sigma = 1 and atomics instead of row sums).
-   The request's quantities are ignored. */
+   The request's quantities are ignored.  The count behind nbl_counts,
+   nbl_row_offsets, nbl_fill and nbl_fill_matrix is made by the first of them
+   called after the forces, on its stream, for the row range and the inputs the
+   forces were computed with. */
 NBL_API nbl_status nbl_lj_forces(nbl_plan *plan, const nbl_request *req, double epsilon,
                                  double sigma, double *forces, double *energy,
                                  void *stream);

@@ -830,7 +830,8 @@ static nbl_status enqueue_build(Plan &p, const Batch &b, bool atoms, int max_run
 static nbl_status enqueue_count_pass(Plan &p, bool ticket_ready, cudaStream_t st) {
     Bufs &B = p.bufs;
     const int64_t N = p.batch_natoms;
-    if (p.i_lo > 0 || p.i_hi < N)
+    // (the build's own row range: the plan's may have been reset since)
+    if (p.targs.i_lo > 0 || p.targs.i_hi < N)
         NBL_CUDA(cudaMemsetAsync(B.counts, 0, sizeof(int32_t) * N, st), "memset counts");
     {
         StageRange r("nbl.count");
@@ -866,8 +867,9 @@ nbl_status enqueue_count(Plan &p, const Batch &b, cudaStream_t st) {
 // calls that read them have them made here.
 static nbl_status ensure_counts(Plan &p, cudaStream_t st) {
     if (!p.count_pending) return NBL_SUCCESS;
-    p.count_pending = false;
-    return enqueue_count_pass(p, false, st);
+    const nbl_status s = enqueue_count_pass(p, false, st);
+    if (s == NBL_SUCCESS) p.count_pending = false;
+    return s;
 }
 
 // What a synchronised count found: its hit-word or list demand, and how its
