@@ -332,6 +332,10 @@ static nbl_status layout_workspace(Plan &p, const Batch &b, int64_t most_list) {
     size_t o_pos32 = L.add(sizeof(float4) * (N + 32));  // read in whole groups of eight
     size_t o_aux = L.add(sizeof(int4) * N);
     size_t o_amax = L.add(sizeof(float) * nsys);
+    // radii in device memory are the caller's: the passes after the gather (a fill
+    // among them, which may come much later) read this copy
+    const bool own_radii = b.per_atom && b.aux_on_device;
+    size_t o_rad = own_radii ? L.add(sizeof(double) * N) : 0;
     size_t o_home = L.add(sizeof(HomeCell) * N);
     size_t o_cnt = L.add(sizeof(int32_t) * (N + 1));
     // row offsets, then the 8-int flag block right after offsets[N]
@@ -388,6 +392,7 @@ static nbl_status layout_workspace(Plan &p, const Batch &b, int64_t most_list) {
     B.pos32 = (float4 *)at(o_pos32);
     B.aux = (int4 *)at(o_aux);
     B.amax = (float *)at(o_amax);
+    B.radius = own_radii ? (double *)at(o_rad) : nullptr;
     B.home = (HomeCell *)at(o_home);
     B.counts = (int32_t *)at(o_cnt);
     B.offsets = (int64_t *)at(o_off);
@@ -691,6 +696,7 @@ static void gather_args(const Plan &p, const Batch &b, const uint32_t *skeys,
     ga.positions = B.pos;
     ga.per_atom = B.per_atom;
     ga.types = B.types;
+    ga.radius = B.radius;
     ga.natoms = b.natoms;
     ga.keys = skeys;
     ga.vals = svals;
@@ -730,7 +736,7 @@ static void traverse_args(Plan &p, const Batch &b, bool atoms, int max_run) {
     ta.pos32 = B.pos32;
     ta.aux = B.aux;
     ta.amax = B.amax;
-    ta.per_atom = B.per_atom;
+    ta.per_atom = B.radius ? B.radius : B.per_atom;
     ta.pt32 = B.pt32;
     ta.pt64 = B.pt64;
     ta.counts = B.counts;

@@ -36,6 +36,7 @@ struct GatherArgs {
     const double *positions;
     const double *per_atom;   // [natoms] or null
     const int32_t *types;     // [natoms] or null
+    double *radius;           // [natoms] copy of per_atom kept by the plan, or null
     int64_t natoms;
     const uint32_t *keys;     // sorted; per atom with skeys
     const int32_t *vals;      // sorted: global atom index; with skeys by cell, any order within
@@ -71,7 +72,7 @@ struct TraverseArgs {
     const float4 *pos32;
     const int4 *aux;
     const float *amax;
-    const double *per_atom;   // [natoms] per-atom radii (original order) or null
+    const double *per_atom;   // [natoms] per-atom radii (original order, the plan's own) or null
     const float *pt32;        // per-type squared cutoffs, FP32
     const double *pt64;       // per-type squared cutoffs, FP64
     int64_t natoms;           // atoms of the batch (offsets[natoms] = pair total)

@@ -63,6 +63,7 @@ struct Bufs {
     double4 *pos64 = nullptr;
     float4 *pos32 = nullptr;
     int4 *aux = nullptr;
+    double *radius = nullptr;      // the plan's copy of the caller's device radii
     float *amax = nullptr;
     HomeCell *home = nullptr;
     int32_t *counts = nullptr;

@@ -143,6 +143,7 @@ __device__ __forceinline__ void gather_one(const GatherArgs &a, int64_t s) {
         if (S.cutoff_kind == kCutPerAtom) {
             const double radius = a.per_atom[at];
             w32 = __double2float_rn(radius);
+            if (a.radius != nullptr) a.radius[at] = radius;
             // (also for NaN and negative radii, whose squares mean nothing)
             if (!(radius >= 0.0 && 2.0 * radius <= S.cutoff)) atomicOr(a.err, kNoteWideRadius);
         } else if (S.cutoff_kind == kCutPerType) {
