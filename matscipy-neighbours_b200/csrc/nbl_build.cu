@@ -56,7 +56,8 @@ namespace nbl {
 __global__ void __launch_bounds__(256)
 k_bin(BinArgs a) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < a.natoms) bin_one(a, t);
+    const unsigned lanes = __ballot_sync(0xffffffffu, t < a.natoms);
+    if (t < a.natoms) bin_one(a, t, lanes);
 }
 
 // ---------------------------------------------------------------------------

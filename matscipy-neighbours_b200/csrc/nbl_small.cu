@@ -81,7 +81,7 @@ k_count_small(SmallCountArgs p) {
     small_sync<CLUSTER>();
 
     // --- bin ----------------------------------------------------------------
-    for (int64_t t = grank; t < N; t += gsize) bin_one(p.bin, t);
+    for (int64_t t = grank; t < N; t += gsize) bin_one(p.bin, t, 0u);  // (not crowded)
     small_sync<CLUSTER>();
 
     // --- stable sort by cell key (CTA 0): bitonic on (key << 32 | atom) ------

@@ -46,8 +46,9 @@ __device__ __forceinline__ uint32_t hash_insert(unsigned long long *hkey,
 }
 
 
-// Atom t (< natoms): its cell key and index for the sort.
-__device__ __forceinline__ void bin_one(const BinArgs &a, int64_t t) {
+// Atom t (< natoms): its cell key and index for the sort.  lanes: the warp's lanes
+// that make this call (read where a.crowded).
+__device__ __forceinline__ void bin_one(const BinArgs &a, int64_t t, unsigned lanes) {
     const int s = a.nsys > 1 ? sys_of(a.sys_atom_base, a.nsys, t) : 0;
     const SysDev &S = a.sys[s];
     double r[3] = {a.positions[3 * t + 0], a.positions[3 * t + 1],
@@ -72,7 +73,7 @@ __device__ __forceinline__ void bin_one(const BinArgs &a, int64_t t) {
     }
     a.keys[t] = key;
     if (a.cell_count != nullptr && a.crowded) {  // one atomic per cell and warp
-        const unsigned peers = __match_any_sync(__activemask(), key);
+        const unsigned peers = __match_any_sync(lanes, key);
         const int lead = __ffs(peers) - 1;
         int first = 0;
         if ((int)(threadIdx.x & 31) == lead)
