@@ -941,6 +941,17 @@ static CountKey count_key(const Plan &p, const Batch &b) {
     k.pos = p.bufs.pos;
     k.per_atom = p.bufs.per_atom;
     k.types = p.bufs.types;
+    k.keys = p.bufs.keys;
+    k.table = p.bufs.table;
+    k.pos64 = p.bufs.pos64;
+    k.offsets = p.bufs.offsets;
+    k.list = p.bufs.list;
+    k.hcell = p.bufs.hcell;
+    k.row_of = p.bufs.row_of;
+    k.end = p.bufs.lj_part;
+    k.row_cap = p.bufs.list_plan.row_cap;
+    k.nvisit = visit_entries(b);
+    k.cull = p.cand_atom > kCullCand ? 1 : 0;
     k.natoms = b.natoms;
     k.table_size = b.table_size;
     k.mask_cap = p.rows ? p.bufs.list_plan.total : p.bufs.mask_cap;

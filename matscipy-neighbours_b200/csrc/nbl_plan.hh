@@ -120,8 +120,10 @@ constexpr double kSparseAtoms = 4.0;
 // constructor zeroes the padding).
 struct CountKey {
     const void *ws_base, *pos, *per_atom, *types;
-    int64_t natoms, table_size, mask_cap, list_chunks, pt_size, i_lo, i_hi;
-    int32_t nsys, grid, key_bits, fp32, kind, itile, max_run, nvisit_tab;
+    // where the layout put the buffers (their sizes shift one another)
+    const void *keys, *table, *pos64, *offsets, *list, *hcell, *row_of, *end;
+    int64_t natoms, table_size, mask_cap, list_chunks, row_cap, pt_size, i_lo, i_hi, nvisit;
+    int32_t nsys, grid, key_bits, fp32, kind, itile, max_run, nvisit_tab, cull;
     int32_t count_mult, count_warps, count_cand, count_group, count_tickets, atoms, sparse;
     CountKey() { std::memset(this, 0, sizeof(*this)); }
     bool operator==(const CountKey &o) const { return std::memcmp(this, &o, sizeof(*this)) == 0; }
