@@ -237,7 +237,8 @@ static double expected_row(const Batch &b, size_t s) {
                                   c[0][1] * (c[1][0] * c[2][2] - c[1][2] * c[2][0]) +
                                   c[0][2] * (c[1][0] * c[2][1] - c[1][1] * c[2][0]));
     const double vol = cell * (double)std::max<int64_t>(b.ncells[s], 1);
-    return (double)S.nat * 4.18879 * S.cutoff * S.cutoff * S.cutoff / std::max(vol, 1e-300);
+    const double rc = std::fabs(S.cutoff);  // (the reference takes negative ones too)
+    return (double)S.nat * 4.18879 * rc * rc * rc / std::max(vol, 1e-300);
 }
 
 // Entries per atom for a mean row of m: room for a uniform system's scatter

@@ -305,7 +305,7 @@ __host__ __device__ __forceinline__ uint32_t morton3(int32_t a, int32_t b, int32
 // reference's exact FP64 arithmetic.
 __host__ __device__ __forceinline__ double guard_band(double M, double R) {
     const double u = 5.9604644775390625e-08;  // 2^-24
-    return 48.0 * u * (M * R + R * R) + 64.0 * u * u * M * M;
+    return 48.0 * u * (M * fabs(R) + R * R) + 64.0 * u * u * M * M;  // (R may be negative)
 }
 
 }  // namespace nbl
