@@ -496,6 +496,19 @@ NBL_API nbl_status nbl_neighbour_list_noalloc(const nbl_request *req,
 #define NBL_INJECT_HASH_CAPACITY 2
 NBL_API nbl_status nbl_debug_inject(int what, int64_t value);
 
+/* What the row passes' lists look like after the last count of a plan or a batch
+   (give one, the other NULL).  For tests.  No reference counterpart. */
+typedef struct nbl_list_info {
+    int64_t workspace_bytes;  /* device workspace held */
+    int64_t list_bytes;       /* room of the lists in it */
+    int lists;                /* 1: the passes go through lists */
+    int by_atoms;             /* 1: counted by one thread per atom, 0: per cell */
+    int two_words;            /* 1: an entry's atom and visit take two words */
+    int short_of_room;        /* 1: some row may have no list (not known before a
+                                 synchronising count) */
+} nbl_list_info;
+NBL_API nbl_status nbl_debug_lists(nbl_plan *plan, nbl_batch *batch, nbl_list_info *info);
+
 /* Last error message of the calling thread ("" if none). */
 NBL_API const char *nbl_last_error(void);
 

@@ -229,7 +229,9 @@ static int64_t mask_words(const Plan &p, const Batch &b) {
     return (int64_t)w;
 }
 
-// Expected neighbours per atom of system s at uniform density.
+// Expected neighbours per atom of system s at uniform density: what the cutoff
+// sphere holds, or the visited cells if that is less (a sheet's or a chain's sphere
+// lies mostly outside an open cell).
 static double expected_row(const Batch &b, size_t s) {
     const SysDev &S = b.sys[s];
     const double(*c)[3] = S.bin;
@@ -238,12 +240,31 @@ static double expected_row(const Batch &b, size_t s) {
                                   c[0][2] * (c[1][0] * c[2][1] - c[1][1] * c[2][0]));
     const double vol = cell * (double)std::max<int64_t>(b.ncells[s], 1);
     const double rc = std::fabs(S.cutoff);  // (the reference takes negative ones too)
-    return (double)S.nat * 4.18879 * rc * rc * rc / std::max(vol, 1e-300);
+    double reach = (double)S.nat;
+    for (int k = 0; k < 3; k++) {
+        const double w = 2.0 * std::max(S.nscan[k], 0) + 1.0;
+        reach *= (S.pbc[k] ? w : std::min(w, (double)S.n[k])) / (double)S.n[k];
+    }
+    return std::min((double)S.nat * 4.18879 * rc * rc * rc / std::max(vol, 1e-300), reach);
+}
+
+// Neighbours that no row of system s exceeds: all atoms, in every image of the cell
+// that its visited offsets touch.
+static double row_limit(const Batch &b, size_t s) {
+    const SysDev &S = b.sys[s];
+    double images = 1.0;
+    for (int k = 0; k < 3; k++)
+        if (S.pbc[k])
+            images *= std::ceil((2.0 * std::max(S.nscan[k], 0) + 1.0) / (double)S.n[k]);
+    return std::max((double)S.nat * images - 1.0, 0.0);
 }
 
 // Entries per atom for a mean row of m: room for a uniform system's scatter
-// (longer rows chain on).
-static double list_entries(double m) { return 1.1 * m + 4.0 * std::sqrt(m) + 4.0; }
+// (longer rows chain on), at most `limit`.
+static double list_entries(double m, double limit) {
+    m = std::min(m, 1e6);
+    return std::min(1.1 * m + 4.0 * std::sqrt(m) + 4.0, limit);
+}
 
 // Sizes of the neighbour lists: every system's entries per atom follow its
 // density, scaled by what the last count of the same sizes found (surfaces,
@@ -264,13 +285,13 @@ static ListPlan plan_lists(const Plan &p, const Batch &b, int64_t most) {
     for (size_t s = 0; s < b.sys.size(); s++) {
         const double m = expected_row(b, s);
         mean += m * (double)b.sys[s].nat;
-        own += list_entries(std::min(scale * m, 1e6)) * (double)b.sys[s].nat;
+        own += list_entries(scale * m, row_limit(b, s)) * (double)b.sys[s].nat;
     }
     lp.expect = mean;
     lp.scale = scale;
     lp.shrink = own > (double)most ? (double)most / own : 1.0;
     int64_t at = 0;
-    for (size_t s = 0; s < b.sys.size(); s++) at += lp.cap(expected_row(b, s)) * b.sys[s].nat;
+    for (size_t s = 0; s < b.sys.size(); s++) at += lp.cap(b, s) * b.sys[s].nat;
     lp.chunks = at;
     const int64_t more = std::min(
         std::max<int64_t>(std::max<int64_t>(at / 4, known ? p.list_hint + p.list_hint / 4 : 0),
@@ -280,8 +301,8 @@ static ListPlan plan_lists(const Plan &p, const Batch &b, int64_t most) {
     lp.row_cap = known && b.natoms > kMarkAtoms ? lp.total * 4 / kRowMark + 16 : 0;
     return lp;
 }
-int64_t ListPlan::cap(double m) const {
-    const double e = list_entries(std::min(scale * m, 1e6)) * shrink;
+int64_t ListPlan::cap(const Batch &b, size_t s) const {
+    const double e = list_entries(scale * expected_row(b, s), row_limit(b, s)) * shrink;
     return (int64_t)std::ceil(e / (wide ? 2.0 : 4.0)) + 1;  // and the link
 }
 
@@ -636,7 +657,7 @@ nbl_status upload_batch(Plan &p, const Batch &b, cudaStream_t st, CountUse use) 
             SysDev *hs = reinterpret_cast<SysDev *>(h);
             int64_t at = 0;
             for (int s2 = 0; s2 < nsys; s2++) {
-                const int64_t cap = B.list_plan.cap(expected_row(b, s2));
+                const int64_t cap = B.list_plan.cap(b, s2);
                 hs[s2].list_base = at;
                 hs[s2].list_cap = (int32_t)cap;
                 at += cap * hs[s2].nat;
@@ -1312,6 +1333,20 @@ nbl_status nbl_set_atom_range(nbl_plan *plan, int64_t lo, int64_t hi) {
                          (long long)lo, (long long)hi);
     plan->p.i_lo = lo;
     plan->p.i_hi = hi;
+    return NBL_SUCCESS;
+}
+
+nbl_status nbl_debug_lists(nbl_plan *plan, nbl_batch *batch, nbl_list_info *info) {
+    clear_error();
+    if (!info || (plan == nullptr) == (batch == nullptr))
+        return set_error(NBL_ERROR_INVALID_ARGUMENT, "one of plan and batch, and info");
+    const Plan &p = plan ? plan->p : batch_plan_of(batch);
+    info->workspace_bytes = (int64_t)p.ws.bytes;
+    info->list_bytes = (int64_t)sizeof(uint4) * p.bufs.list_plan.total;
+    info->lists = p.rows ? 1 : 0;
+    info->by_atoms = p.sparse ? 1 : 0;
+    info->two_words = p.bufs.list_plan.wide ? 1 : 0;
+    info->short_of_room = p.lists_short ? 1 : 0;
     return NBL_SUCCESS;
 }
 

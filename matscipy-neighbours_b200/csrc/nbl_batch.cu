@@ -128,6 +128,8 @@ struct nbl_batch {
     float tuned_fill_ms = 0.f;
 };
 
+const Plan &nbl::batch_plan_of(const nbl_batch *bt) { return bt->p; }
+
 namespace {
 
 struct Guard {

@@ -40,7 +40,7 @@ struct ListPlan {
     int64_t row_cap = 0;            // row marks
     double expect = 0.0;            // pairs the density alone would give
     double scale = 1.0, shrink = 1.0;
-    int64_t cap(double expected_row) const;  // groups per atom
+    int64_t cap(const Batch &b, size_t system) const;  // groups per atom
 };
 
 // Device buffers of one call, carved out of the workspace.
@@ -235,6 +235,7 @@ nbl_status plan_system(const double origin[3], const double cell[9],
                        SysDev &S, int64_t &ncells);
 nbl_status finish_batch(Batch &b, int grid_req);
 nbl_status upload_batch(Plan &p, const Batch &b, cudaStream_t st, CountUse use = kUseLists);
+const Plan &batch_plan_of(const nbl_batch *bt);
 void note_lists(Plan &p, const Batch &b, int64_t npairs, int64_t demand, int flags);
 nbl_status enqueue_count(Plan &p, const Batch &b, cudaStream_t st);
 nbl_status run_count(Plan &p, const Batch &b, cudaStream_t st, bool sync);
