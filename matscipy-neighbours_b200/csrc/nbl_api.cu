@@ -266,36 +266,54 @@ static double list_entries(double m, double limit) {
     return std::min(1.1 * m + 4.0 * std::sqrt(m) + 4.0, limit);
 }
 
-// Sizes of the neighbour lists: every system's entries per atom follow its
-// density, scaled by what the last count of the same sizes found (surfaces,
-// cutoffs below the widest); a quarter on top, or what the last count took
-// and more, for chained chunks; at most about `most` entries.
+// Rows of system s that the plan's row range asks for: how many, and the first one
+// (an atom of the system).
+static int64_t listed_rows(const Plan &p, const Batch &b, size_t s, int64_t &first) {
+    const SysDev &S = b.sys[s];
+    const int64_t base = S.atom_base, end = base + S.nat;
+    const int64_t lo = std::min(std::max(p.i_lo, base), end);
+    first = lo - base;
+    return std::max<int64_t>(std::min(p.i_hi, end) - lo, 0);
+}
+
+// Whether p's learned list sizes are those of batch b and the plan's row range.
+static bool lists_known(const Plan &p, const Batch &b) {
+    return p.list_natoms == b.natoms && p.list_table == b.table_size && p.list_lo == p.i_lo &&
+           p.list_hi == p.i_hi;
+}
+
+// Sizes of the neighbour lists of the rows in range: every system's entries per
+// atom follow its density, or, if that is more, the pairs that a count of the same
+// sizes found; on top a quarter, or what such a count took and more, for chained
+// chunks; at most about `most` entries.
 static ListPlan plan_lists(const Plan &p, const Batch &b, int64_t most) {
     ListPlan lp;
-    const bool known =
-        !p.forces && p.list_natoms == b.natoms && p.list_table == b.table_size;
+    const bool known = !p.forces && lists_known(p, b);
+    int64_t first = 0;
+    double mean = 0.0;
+    for (size_t s = 0; s < b.sys.size(); s++)
+        mean += expected_row(b, s) * (double)listed_rows(p, b, s, first);
+    lp.expect = mean;
     // (a force pass writes no lists: should the list be asked for afterwards, most
     // rows run out of room and the thread-per-atom fill writes them)
-    const double scale = p.forces ? 0.0 : known ? p.list_scale : 1.0;
+    const double scale =
+        p.forces ? 0.0 : known && mean > 0.0 ? std::max(p.list_pairs / mean, 1.0) : 1.0;
     int max_visit = 0;
     for (const SysDev &S : b.sys) max_visit = std::max(max_visit, S.nvisit);
     lp.shift = 32 - bits_for((uint64_t)std::max(max_visit - 1, 1));
     lp.wide = b.natoms > (int64_t(1) << lp.shift);
-    double own = 0.0, mean = 0.0;
-    for (size_t s = 0; s < b.sys.size(); s++) {
-        const double m = expected_row(b, s);
-        mean += m * (double)b.sys[s].nat;
-        own += list_entries(scale * m, row_limit(b, s)) * (double)b.sys[s].nat;
-    }
-    lp.expect = mean;
+    double own = 0.0;
+    for (size_t s = 0; s < b.sys.size(); s++)
+        own += list_entries(scale * expected_row(b, s), row_limit(b, s)) *
+               (double)listed_rows(p, b, s, first);
     lp.scale = scale;
     lp.shrink = own > (double)most ? (double)most / own : 1.0;
     int64_t at = 0;
-    for (size_t s = 0; s < b.sys.size(); s++) at += lp.cap(b, s) * b.sys[s].nat;
+    for (size_t s = 0; s < b.sys.size(); s++)
+        at += lp.cap(b, s) * listed_rows(p, b, s, first);
     lp.chunks = at;
     const int64_t more = std::min(
-        std::max<int64_t>(std::max<int64_t>(at / 4, known ? p.list_hint + p.list_hint / 4 : 0),
-                          int64_t(1) << 16),
+        std::max<int64_t>(std::max<int64_t>(at / 4, known ? p.list_more : 0), int64_t(1) << 16),
         most / 4);
     lp.total = at + more;
     lp.row_cap = known && b.natoms > kMarkAtoms ? lp.total * 4 / kRowMark + 16 : 0;
@@ -657,10 +675,13 @@ nbl_status upload_batch(Plan &p, const Batch &b, cudaStream_t st, CountUse use) 
             SysDev *hs = reinterpret_cast<SysDev *>(h);
             int64_t at = 0;
             for (int s2 = 0; s2 < nsys; s2++) {
+                // (lists of the rows in range only, of which `first` is the first)
                 const int64_t cap = B.list_plan.cap(b, s2);
-                hs[s2].list_base = at;
+                int64_t first = 0;
+                const int64_t rows = listed_rows(p, b, s2, first);
+                hs[s2].list_base = at - first * cap;
                 hs[s2].list_cap = (int32_t)cap;
-                at += cap * hs[s2].nat;
+                at += cap * rows;
             }
         }
         if (B.visit != nullptr) {
@@ -900,19 +921,30 @@ static nbl_status ensure_counts(Plan &p, cudaStream_t st) {
     return s;
 }
 
-// What a synchronised count found: its hit-word or list demand, and how its
-// pairs compare with the density's estimate.
+// What a synchronised count found: its hit-word or list demand, and its pairs.
+// List sizes only grow while the plan's calls have the same sizes, and in steps:
+// calls that take turns (another density, other cutoffs) neither shorten one
+// another's lists nor change the layout, which the captured count phase depends on,
+// each time.
 void note_lists(Plan &p, const Batch &b, int64_t npairs, int64_t demand, int flags) {
     p.lists_short = (flags & kErrNoList) != 0;
     if (!p.rows) {
         p.mask_hint = demand;
         return;
     }
-    p.list_natoms = b.natoms;
-    p.list_table = b.table_size;
-    p.list_hint = demand;
-    const double e = p.bufs.list_plan.expect;
-    p.list_scale = e > 0.0 ? std::min((double)npairs / e, 1e3) : 1.0;
+    if (!lists_known(p, b)) {
+        p.list_natoms = b.natoms;
+        p.list_table = b.table_size;
+        p.list_lo = p.i_lo;
+        p.list_hi = p.i_hi;
+        p.list_pairs = 0.0;
+        p.list_more = 0;
+    }
+    const ListPlan &lp = p.bufs.list_plan;
+    const int64_t more = lp.total - lp.chunks;
+    if (demand <= more - more / 8) return;
+    if ((double)npairs > lp.scale * lp.expect) p.list_pairs = 1.0625 * (double)npairs;
+    p.list_more = (demand + demand / 4 + 4095) & ~int64_t(4095);
 }
 
 // Whether batch b takes the one-launch count phase (nbl_small.cu): one system of

@@ -92,7 +92,8 @@ struct SysDev {
     int32_t pt_base;     // first entry of this system's per-type tables
     int32_t nvisit;      // (2nx+1)(2ny+1)(2nz+1)
     int64_t visit_base;  // first VisitDev entry of this system, -1: computed per item
-    int64_t list_base;   // neighbour lists (nbl_rows.cu): first group of this system,
+    int64_t list_base;   // neighbour lists (nbl_rows.cu): first group of this system's atom
+                         // 0 (negative where only later rows have lists), and
     int32_t list_cap;    // groups per atom (the last one is the link)
     int32_t pad_;
 };

@@ -171,16 +171,16 @@ struct Plan {
     bool count_tickets = true;
     bool fill_tickets = true;
     int64_t mask_hint = 0;    // mask-pool words the last count asked for
-    // Row passes in use; and what the last synchronised count of these sizes
-    // found: chained entries, pairs against the density's estimate.
+    // Row passes in use; and what the synchronised counts of these sizes found.
     bool rows = false;
     double cand_atom = 0.0;   // atoms of the cells that an atom visits, on average
     bool forces = false;      // a force pass: no lists planned
     bool sparse = false;      // with one thread per atom in the count
     bool spare_ticket = false;  // a cleared work-item ticket is left for one fill
     bool lists_short = true;  // some row may have no list (kErrNoList)
-    int64_t list_natoms = -1, list_table = -1, list_hint = 0;
-    double list_scale = 1.0;
+    // (the sizes: atoms, table, row range; groups of chained chunks to plan for)
+    int64_t list_natoms = -1, list_table = -1, list_lo = 0, list_hi = 0, list_more = 0;
+    double list_pairs = 0.0;
     // Row range of nbl_set_atom_range (global atom indices, [lo, hi)).
     int64_t i_lo = 0;
     int64_t i_hi = INT64_MAX;

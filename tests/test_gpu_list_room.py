@@ -38,3 +38,60 @@ def test_open_systems_of_every_shape(oracle, n, shape, cutoff):
         assert info.lists and not info.short_of_room
         # an entry is 4 bytes; a MB for chains, and the scatter of short rows
         assert info.list_bytes <= 8 * len(want[0]) + 400 * n + (2 << 20)
+
+
+def _bulk(n=20000, seed=0):
+    rng = np.random.default_rng(seed)
+    box = (n / 0.085) ** (1.0 / 3.0)
+    cell = box * np.array([[1.0, 0.0, 0.0], [0.1, 1.0, 0.0], [0.0, -0.2, 1.0]])
+    return np.ascontiguousarray(rng.uniform(size=(n, 3)) @ cell), cell
+
+
+def test_rows_of_a_range_and_full_lists_in_turn(oracle):
+    """A range's lists hold its rows only, and a call of one range leaves the next
+    call of another one with all the room it needs."""
+    import torch
+    from matscipy_neighbours.distributed import neighbour_list_rows
+    pos, cell = _bulk()
+    pbc = np.array([True, True, False])
+    want = oracle.oracle_neighbour_list("ijdDS", cell, pos, 4.0, pbc)
+    dev = torch.from_numpy(pos).cuda()
+    plan = _plan()
+    room = {}
+    for rows in ((0, 20000), (5000, 7500), (0, 20000), (5000, 7500), (0, 2500), (19999, 20000),
+                 (0, 20000), (17, 17)):
+        got = neighbour_list_rows("ijdDS", dev, cell, pbc, 4.0, rows)
+        torch.cuda.synchronize()
+        keep = (want[0] >= rows[0]) & (want[0] < rows[1])
+        assert_same_lists(tuple(g.cpu().numpy() for g in got), tuple(w[keep] for w in want),
+                          "ijdDS")
+        info = list_info(plan)
+        assert not info.short_of_room, rows
+        assert room.setdefault(rows, info.list_bytes) == info.list_bytes, rows
+    own = lambda rows: room[rows] - (1 << 20)   # (a MB for chains)
+    assert own((5000, 7500)) < own((0, 20000)) / 6
+
+
+def test_cutoff_kinds_and_densities_in_turn(oracle):
+    """Few pairs, then many, of the same sizes: no call's room follows the other's."""
+    from matscipy_neighbours import neighbour_list
+    pos, cell = _bulk(n=6000)
+    rng = np.random.default_rng(4)
+    types = rng.integers(0, 2, size=6000).astype(np.int32)
+    few = np.array([[4.0, 1.0], [1.0, 1.0]])
+    types[:] = 1
+    types[0] = 0
+    squeezed = pos.copy()
+    squeezed[:, 0] *= 0.3
+    pbc = np.array([True, False, True])
+    calls = [(pos, few, types), (pos, 4.0, None), (squeezed, 4.0, None), (pos, few, types),
+             (squeezed, 4.0, None), (pos, 4.0, None)]
+    plan = _plan()
+    sizes = []
+    for p, cut, ty in calls + calls:
+        want = oracle.oracle_neighbour_list("ijdDS", cell, p, cut, pbc, types=ty)
+        got = neighbour_list("ijdDS", positions=p, cell=cell, pbc=pbc, cutoff=cut, numbers=ty)
+        assert_same_lists(got, want, "ijdDS")
+        sizes.append(list_info(plan).list_bytes)
+    assert len(set(sizes[len(calls):])) == 1, sizes
+    assert not list_info(plan).short_of_room
