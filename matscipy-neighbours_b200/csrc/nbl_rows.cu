@@ -52,13 +52,14 @@ constexpr int kSplitBuf = 16;  // list entries a lane of those buffers
 template <bool WIDE>
 struct RowList {
     uint4 q;
-    long long wp;  // next group
+    long long wp;  // next group; without a list any more, the groups it holds
     int room;      // groups left before the link; -1: no list any more
     int n;         // row length
     __device__ __forceinline__ void put(const TraverseArgs &a) {
         if (room == 0) {
-            wp = list_grow(a, wp);
-            room = wp >= 0 ? kListChunk - 1 : -1;
+            const long long next = list_grow(a, wp);
+            room = next >= 0 ? kListChunk - 1 : -1;
+            wp = next >= 0 ? next : (n - 1) / Entry<WIDE>::kPerGroup;
         }
         if (room > 0) {
             a.list[wp] = q;
@@ -92,6 +93,7 @@ struct RowList {
     }
     __device__ __forceinline__ void finish(const TraverseArgs &a) {
         if (n & (Entry<WIDE>::kPerGroup - 1)) put(a);
+        if (room < 0) list_lacks(a, n - wp * Entry<WIDE>::kPerGroup, Entry<WIDE>::kPerGroup);
     }
 };
 

@@ -43,7 +43,8 @@ struct __align__(16) ListWarp {
     uint16_t code[kListCand];   // hits of the atoms in hand, in order: staged candidates
     float4 i32[kITile];
     long long lw[kITile];       // entry index of rank 0, as if the current segment began there
-    int32_t lim[kITile];        // first rank beyond the segment; -1: no list any more
+    int32_t lim[kITile];        // first rank beyond the segment; -1: no list any more (lw: the
+                                // entries it holds)
     int32_t icount[kITile];     // row lengths so far
     int32_t iatom[kITile];
     int32_t isi[kITile];
@@ -246,6 +247,7 @@ __device__ __forceinline__ void list_emit(ListWarp<WIDE> &sm, const TraverseArgs
                         const long long next = list_grow(a, (lw + lim) / E::kPerGroup);
                         if (next < 0) {
                             sm.lim[ilh] = -1;
+                            sm.lw[ilh] = lim;
                         } else {
                             sm.lw[ilh] = next * E::kPerGroup - lim;
                             sm.lim[ilh] = lim + (kListChunk - 1) * E::kPerGroup;
@@ -546,6 +548,7 @@ k_count_list(const __grid_constant__ TraverseArgs a) {
             }
         } else if (lane < ni) {
             a.counts[sm.iatom[lane]] = sm.icount[lane];
+            if (sm.lim[lane] < 0) list_lacks(a, sm.icount[lane] - sm.lw[lane], E::kPerGroup);
         }
         __syncwarp();
         L.step();

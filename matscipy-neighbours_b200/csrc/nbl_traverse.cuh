@@ -160,6 +160,14 @@ __device__ __noinline__ long long list_grow(const TraverseArgs &a, long long at)
     return (long long)next;
 }
 
+// A row that found no chunk keeps `rest` entries outside its list: the other chunks
+// it would have taken are asked for too, so that the cursor ends as the whole demand.
+__device__ __forceinline__ void list_lacks(const TraverseArgs &a, long long rest, int per_group) {
+    const long long in = (kListChunk - 1) * per_group;
+    const long long more = (rest + in - 1) / in - 1;
+    if (more > 0) atomicAdd(a.mask_cursor, (unsigned long long)(more * kListChunk));
+}
+
 template <bool FP32, int CAND>
 struct __align__(16) CountSmem {
     SegSmem sg;

@@ -95,3 +95,35 @@ def test_cutoff_kinds_and_densities_in_turn(oracle):
         sizes.append(list_info(plan).list_bytes)
     assert len(set(sizes[len(calls):])) == 1, sizes
     assert not list_info(plan).short_of_room
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("place", ["droplet", "blob", "half"])
+@pytest.mark.parametrize("n", [300, 2500])
+def test_first_count_of_crowded_atoms_has_room(oracle, n, place, precision):
+    """Atoms crowded into a small part of their box, where the mean density lets expect
+    hardly any neighbours: every row has its list after the first call already."""
+    from matscipy_neighbours import _matscipy_neighbours as ext
+    from matscipy_neighbours import neighbour_list
+    rng = np.random.default_rng(n)
+    cell = np.diag([120.0, 130.0, 110.0])
+    u = rng.uniform(size=(n, 3))
+    if place == "droplet":
+        pos = 50.0 + u * (n / 0.08) ** (1.0 / 3.0)
+    else:
+        pos = 50.0 + u
+        if place == "half":
+            pos[::2] = u[::2] @ cell
+    pbc = np.array([False] * 3)
+    want = oracle.oracle_neighbour_list("ijdDS", cell, pos, 3.0, pbc)
+    plan = _plan()
+    neighbour_list("i", positions=u[:200] * 20.0, cell=cell, pbc=pbc, cutoff=3.0)  # other sizes
+    prev = ext.set_options(precision=precision)
+    try:
+        for _ in range(2):
+            got = neighbour_list("ijdDS", positions=pos, cell=cell, pbc=pbc, cutoff=3.0)
+            assert_same_lists(got, want, "ijdDS")
+            info = list_info(plan)
+            assert info.lists and not info.short_of_room
+    finally:
+        ext.set_options(**prev)
