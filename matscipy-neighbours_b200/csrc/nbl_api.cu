@@ -602,10 +602,13 @@ static bool atom_mode(const Plan &p, const Batch &b) {
 }
 
 // Whether the count takes one thread per atom (nbl_rows.cu) instead of one warp
-// per cell: where the occupied cells hold few atoms.
+// per cell: where the occupied cells hold few atoms, and the atoms have no more
+// neighbours than such cells give (a blob in a gas leaves the mean per cell small, but
+// its one cell is where the time goes: 1,500 atoms of each, 780 us by atoms, 410 per cell).
 static bool sparse_grid(const Plan &p, const Batch &b) {
     if (p.occ_cells > 0 && p.occ_natoms == b.natoms && p.occ_table == b.table_size)
-        return (double)b.natoms < kSparseAtoms * (double)p.occ_cells;
+        return (double)b.natoms < kSparseAtoms * (double)p.occ_cells &&
+               (double)p.occ_pairs < 4.18879 * kSparseAtoms * (double)b.natoms;
     double cells = 0.0;
     for (int64_t n : b.ncells) cells += (double)n;
     return (double)b.natoms < kSparseAtoms * cells;
@@ -1132,6 +1135,7 @@ static nbl_status count_once(Plan &p, const Batch &b, cudaStream_t st, bool sync
             p.occ_natoms = N;
             p.occ_table = b.table_size;
             p.occ_cells = flags[0];
+            p.occ_pairs = p.npairs;
         }
         unsigned long long demand = 0;  // mask-pool words the count asked for
         std::memcpy(&demand, flags + 4, sizeof(demand));

@@ -164,9 +164,9 @@ struct Plan {
     // occupied cells hold fewer than two atoms on average, -1 = never, 1 =
     // always (where the systems have visit tables).
     int atom_threads = 0;
-    // Occupied cells counted by the last synchronised count, with the atom
-    // count and table size it ran on (steers the default choice above).
-    int64_t occ_natoms = -1, occ_table = -1, occ_cells = 0;
+    // Occupied cells and pairs counted by the last synchronised count, with the
+    // atom count and table size it ran on (steers the default choices).
+    int64_t occ_natoms = -1, occ_table = -1, occ_cells = 0, occ_pairs = 0;
     // Work items by atomic ticket (else a fixed warp stride) in each pass.
     bool count_tickets = true;
     bool fill_tickets = true;

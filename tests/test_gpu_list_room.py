@@ -127,3 +127,20 @@ def test_first_count_of_crowded_atoms_has_room(oracle, n, place, precision):
             assert info.lists and not info.short_of_room
     finally:
         ext.set_options(**prev)
+
+
+@pytest.mark.parametrize("blob,by_atoms", [(0, 1), (1500, 0)])
+def test_a_blob_in_a_gas_is_counted_by_cells(oracle, blob, by_atoms):
+    """Few atoms per occupied cell on average, but most pairs in one cell."""
+    from matscipy_neighbours import neighbour_list
+    rng = np.random.default_rng(blob)
+    cell = 100.0 * np.eye(3)
+    pos = rng.uniform(size=(3000, 3)) @ cell
+    pos[:blob] = 50.0 + rng.uniform(size=(blob, 3))
+    pbc = np.array([False, True, False])
+    want = oracle.oracle_neighbour_list("ijdDS", cell, pos, 2.5, pbc)
+    plan = _plan()
+    for _ in range(3):
+        got = neighbour_list("ijdDS", positions=pos, cell=cell, pbc=pbc, cutoff=2.5)
+        assert_same_lists(got, want, "ijdDS")
+    assert list_info(plan).by_atoms == by_atoms
