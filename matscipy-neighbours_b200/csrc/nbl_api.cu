@@ -928,6 +928,16 @@ static nbl_status ensure_counts(Plan &p, cudaStream_t st) {
     return s;
 }
 
+// What a synchronised count found, for the next call's choice of passes: occupied
+// cells and pairs.
+void note_count(Plan &p, const Batch &b, int64_t npairs, int occupied) {
+    if (occupied <= 0) return;
+    p.occ_natoms = b.natoms;
+    p.occ_table = b.table_size;
+    p.occ_cells = occupied;
+    p.occ_pairs = npairs;
+}
+
 // What a synchronised count found: its hit-word or list demand, and its pairs.
 // List sizes only grow while the plan's calls have the same sizes, and in steps:
 // calls that take turns (another density, other cutoffs) neither shorten one
@@ -1131,12 +1141,7 @@ static nbl_status count_once(Plan &p, const Batch &b, cudaStream_t st, bool sync
         int flags[6];
         std::memcpy(flags, p.host_small + 1, sizeof(flags));
         p.npairs = p.host_small[0];
-        if (flags[0] > 0) {  // occupied cells, for the next call's choice of passes
-            p.occ_natoms = N;
-            p.occ_table = b.table_size;
-            p.occ_cells = flags[0];
-            p.occ_pairs = p.npairs;
-        }
+        note_count(p, b, p.npairs, flags[0]);
         unsigned long long demand = 0;  // mask-pool words the count asked for
         std::memcpy(&demand, flags + 4, sizeof(demand));
         note_lists(p, b, p.npairs, (int64_t)demand, flags[1]);

@@ -531,23 +531,30 @@ NBL_API nbl_status nbl_batch_setup(nbl_batch *bt, const nbl_batch_request *req,
     if (s != NBL_SUCCESS) return s;
     NBL_CUDA(cudaStreamSynchronize(st), "batch upload");
     bt->p.stage_in_flight = false;
-    // Capacity: measured when not given (25 % headroom for later steps).
-    if (capacity <= 0) {
+    // Capacity: measured when not given (25 % headroom for later steps); so is the
+    // lists' room, which a given capacity says nothing about.
+    if (capacity <= 0 || bt->p.rows) {
         s = enqueue_count(bt->p, b, st);
         if (s != NBL_SUCCESS) return s;
         NBL_CUDA(cudaMemcpyAsync(bt->p.host_small, bt->p.bufs.offsets + N,
                                  sizeof(int64_t) + sizeof(int) * 6, cudaMemcpyDeviceToHost, st),
                  "read pair count and mask demand");
         NBL_CUDA(cudaStreamSynchronize(st), "count");
-        capacity = bt->p.host_small[0] + bt->p.host_small[0] / 4 + 4096;
-        // More hit words asked for than the estimate held: re-plan the
-        // workspace with the measured demand before the graph is captured.
+        const int64_t npairs = bt->p.host_small[0];
+        if (capacity <= 0) capacity = npairs + npairs / 4 + 4096;
+        // More list room or hit words asked for than the estimate held: re-plan
+        // the workspace with the measured demand before the graph is captured.
+        // (Flagged errors come back from the first run; such a count says nothing.)
         int flags[6];
         std::memcpy(flags, bt->p.host_small + 1, sizeof(flags));
         unsigned long long demand = 0;
         std::memcpy(&demand, flags + 4, sizeof(demand));
-        note_lists(bt->p, b, bt->p.host_small[0], (int64_t)demand, flags[1]);
-        if (bt->p.rows || (long long)demand > bt->p.bufs.mask_cap) {
+        const bool good = !(flags[1] & (kErrRange | kErrInternal));
+        if (good) {
+            note_count(bt->p, b, npairs, flags[0]);
+            note_lists(bt->p, b, npairs, (int64_t)demand, flags[1]);
+        }
+        if (good && (bt->p.rows || (long long)demand > bt->p.bufs.mask_cap)) {
             s = upload_batch(bt->p, b, st);
             if (s != NBL_SUCCESS) return s;
             NBL_CUDA(cudaStreamSynchronize(st), "batch upload");

@@ -236,6 +236,7 @@ nbl_status plan_system(const double origin[3], const double cell[9],
 nbl_status finish_batch(Batch &b, int grid_req);
 nbl_status upload_batch(Plan &p, const Batch &b, cudaStream_t st, CountUse use = kUseLists);
 const Plan &batch_plan_of(const nbl_batch *bt);
+void note_count(Plan &p, const Batch &b, int64_t npairs, int occupied);
 void note_lists(Plan &p, const Batch &b, int64_t npairs, int64_t demand, int flags);
 nbl_status enqueue_count(Plan &p, const Batch &b, cudaStream_t st);
 nbl_status run_count(Plan &p, const Batch &b, cudaStream_t st, bool sync);

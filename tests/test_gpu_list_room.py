@@ -144,3 +144,27 @@ def test_a_blob_in_a_gas_is_counted_by_cells(oracle, blob, by_atoms):
         got = neighbour_list("ijdDS", positions=pos, cell=cell, pbc=pbc, cutoff=2.5)
         assert_same_lists(got, want, "ijdDS")
     assert list_info(plan).by_atoms == by_atoms
+
+
+@pytest.mark.parametrize("capacity", [None, 3 << 20])
+def test_batch_of_droplets_has_room(oracle, capacity):
+    """The lists of a batch are sized by a count, also where the caller gives the
+    output's capacity."""
+    from matscipy_neighbours.batch import NeighbourListBatch
+    rng = np.random.default_rng(2)
+    cell = 90.0 * np.eye(3)
+    systems = [dict(positions=40.0 + rng.uniform(size=(n, 3)) * w, cell=cell,
+                    pbc=np.array([False, True, False]), cutoff=3.0)
+               for n, w in ((600, 2.0), (1500, 25.0), (3, 1.0), (400, 1.0))]
+    b = NeighbourListBatch(systems, autotune=False, capacity=capacity)
+    for _ in range(2):
+        b.run()
+        off = b.sys_offsets()
+        outs = [t.cpu().numpy() for t in b.results()]
+        for s, sd in enumerate(systems):
+            want = oracle.oracle_neighbour_list("ijdDS", cell, sd["positions"], 3.0, sd["pbc"])
+            assert_same_lists(tuple(o[off[s]:off[s + 1]] for o in outs), want, "ijdDS")
+    info = list_info(batch=b._h)
+    assert info.lists and not info.by_atoms
+    assert info.list_bytes >= 4 * off[-1]
+    b.close()
