@@ -390,20 +390,7 @@ template <bool WIDE>
 __device__ __forceinline__ bool list_entry(const TraverseArgs &a, long long base, int cap,
                                            long long r, int &sj, int &v) {
     using E = Entry<WIDE>;
-    if (r >= cap) {
-        constexpr int kIn = (kListChunk - 1) * E::kPerGroup;  // entries of a chunk
-        long long link = base + cap / E::kPerGroup;
-        r -= cap;
-        while (true) {
-            const uint4 l = a.list[link];
-            if (l.x == kNoLink && l.y == kNoLink) return false;
-            base = (long long)((unsigned long long)l.x | (unsigned long long)l.y << 32);
-            if (checked_fail(base < 0 || base + kListChunk > a.list_cap, a.err)) return false;
-            if (r < kIn) break;
-            link = base + kListChunk - 1;
-            r -= kIn;
-        }
-    }
+    if (!list_reach<WIDE>(a, base, cap, r)) return false;
     E::get(a.list_shift, reinterpret_cast<const typename E::T *>(a.list + base)[r], sj, v);
     return !checked_fail(sj < 0 || sj >= a.natoms, a.err);
 }

@@ -152,6 +152,14 @@ __device__ __forceinline__ void emit_pair(const TraverseArgs &a, const Hot &H, c
     }
 }
 
+// Whether atom si's row (atom at) was written from its list.
+template <bool WIDE>
+__device__ __forceinline__ bool row_listed(const TraverseArgs &a, int64_t si, int32_t at) {
+    const SysDev &S = a.sys[a.hcell[si].w];
+    long long base = S.list_base + (at - S.atom_base) * S.list_cap, last = a.counts[at] - 1ll;
+    return list_reach<WIDE>(a, base, (S.list_cap - 1) * Entry<WIDE>::kPerGroup, last);
+}
+
 // One sorted atom's row: its length (FILL = false, into counts) or its pairs
 // (FILL = true, at offsets[i] on).  ALL5: all five outputs, no matrix.
 template <int KIND, bool FILL, bool ALL5>
@@ -161,8 +169,8 @@ __device__ __forceinline__ void atom_row(const TraverseArgs &a, int64_t si) {
     const int4 ai = a.aux[si];
     if (checked_fail(ai.x < 0 || ai.x >= a.natoms, a.err)) return;
     if (ai.x < a.i_lo || ai.x >= a.i_hi) return;
-    if (FILL && a.list != nullptr && 
-        a.counts[ai.x] <= (a.sys[a.hcell[si].w].list_cap - 1) * (a.list_wide ? 2 : 4))
+    if (FILL && a.list != nullptr &&
+        (a.list_wide ? row_listed<true>(a, si, ai.x) : row_listed<false>(a, si, ai.x)))
         return;
     int sys = 0;
     int32_t cc[3] = {0, 0, 0};

@@ -160,6 +160,27 @@ __device__ __noinline__ long long list_grow(const TraverseArgs &a, long long at)
     return (long long)next;
 }
 
+// Follows a row's list (first group `base`, `cap` entries before the chain) to entry
+// r: its segment's first group in base, its place there in r; false when the row has
+// no list that far.
+template <bool WIDE>
+__device__ __forceinline__ bool list_reach(const TraverseArgs &a, long long &base, int cap,
+                                           long long &r) {
+    if (r < cap) return true;
+    constexpr int kIn = (kListChunk - 1) * Entry<WIDE>::kPerGroup;  // entries of a chunk
+    long long link = base + cap / Entry<WIDE>::kPerGroup;
+    r -= cap;
+    while (true) {
+        const uint4 l = a.list[link];
+        if (l.x == kNoLink && l.y == kNoLink) return false;
+        base = (long long)((unsigned long long)l.x | (unsigned long long)l.y << 32);
+        if (checked_fail(base < 0 || base + kListChunk > a.list_cap, a.err)) return false;
+        if (r < kIn) return true;
+        link = base + kListChunk - 1;
+        r -= kIn;
+    }
+}
+
 // A row that found no chunk keeps `rest` entries outside its list: the other chunks
 // it would have taken are asked for too, so that the cursor ends as the whole demand.
 __device__ __forceinline__ void list_lacks(const TraverseArgs &a, long long rest, int per_group) {
