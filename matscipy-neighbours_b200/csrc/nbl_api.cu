@@ -285,6 +285,15 @@ static bool lists_known(const Plan &p, const Batch &b) {
            p.list_hi == p.i_hi;
 }
 
+// Entries that the lists of batch b may have: what the device had room for when a call
+// of these sizes last asked for more than there was.
+static int64_t list_limit(const Plan &p, const Batch &b) {
+    return p.most_natoms == b.natoms && p.most_table == b.table_size && p.most_lo == p.i_lo &&
+                   p.most_hi == p.i_hi
+               ? p.list_most
+               : kMostList;
+}
+
 // Sizes of the neighbour lists of the rows in range: every system's entries per
 // atom follow its density, or, if that is more, the pairs that a count of the same
 // sizes found; on top a quarter, or what such a count took and more, for chained
@@ -454,15 +463,25 @@ static nbl_status layout_workspace(Plan &p, const Batch &b, int64_t most_list) {
 }
 
 // The same with lists for every expected pair or, where the device has no room for
-// them, few: rows without room are written by the thread-per-atom fill.
+// them, an eighth, and so on: rows without room are written by the thread-per-atom
+// fill.  What the device had room for is remembered for these sizes: a call that asks
+// for more releases the workspace first, and on a full device would each time.
 static nbl_status layout_workspace(Plan &p, const Batch &b) {
-    constexpr int64_t kFew = int64_t(1) << 26;
-    const nbl_status st = layout_workspace(p, b, kMostList);
-    if (st != NBL_ERROR_OUT_OF_MEMORY || !p.rows ||
-        4 * plan_lists(p, b, kMostList).total <= kFew)
-        return st;
-    clear_error();
-    return layout_workspace(p, b, kFew);
+    constexpr int64_t kFew = int64_t(1) << 18;
+    while (true) {
+        const int64_t most = list_limit(p, b);
+        const nbl_status st = layout_workspace(p, b, most);
+        if (st != NBL_ERROR_OUT_OF_MEMORY || !p.rows) return st;
+        const int64_t now = 4 * plan_lists(p, b, most).total;
+        const int64_t less = std::max(now / 8, kFew);
+        if (2 * 4 * plan_lists(p, b, less).total > now) return st;  // not the lists
+        clear_error();
+        p.most_natoms = b.natoms;
+        p.most_table = b.table_size;
+        p.most_lo = p.i_lo;
+        p.most_hi = p.i_hi;
+        p.list_most = less;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -956,7 +975,9 @@ void note_lists(Plan &p, const Batch &b, int64_t npairs, int64_t demand, int fla
         p.list_hi = p.i_hi;
         p.list_pairs = 0.0;
         p.list_more = 0;
+        p.list_stay = false;
     }
+    if (p.list_stay) return;
     const ListPlan &lp = p.bufs.list_plan;
     const int64_t more = lp.total - lp.chunks;
     if (demand <= more - more / 8) return;
@@ -1091,7 +1112,7 @@ static bool capture_count(Plan &p, const Batch &b, const CountKey &k) {
 
 // Whether lists planned now would have more room than those of the last count.
 static bool lists_can_grow(const Plan &p, const Batch &b) {
-    return plan_lists(p, b, kMostList).total > p.bufs.list_plan.total;
+    return !p.list_stay && plan_lists(p, b, list_limit(p, b)).total > p.bufs.list_plan.total;
 }
 
 static nbl_status count_once(Plan &p, const Batch &b, cudaStream_t st, bool sync) {
@@ -1161,8 +1182,15 @@ static nbl_status count_once(Plan &p, const Batch &b, cudaStream_t st, bool sync
 // calls with two counts / with those rows: droplets of 100,000 and 200,000 atoms in a
 // box four times as wide 780 / 990 and 1,090 / 1,610 us.
 nbl_status run_count(Plan &p, const Batch &b, cudaStream_t st, bool sync) {
-    const nbl_status s = count_once(p, b, st, sync);
+    nbl_status s = count_once(p, b, st, sync);
     if (s != NBL_SUCCESS || !sync || !p.rows || !p.lists_short || !lists_can_grow(p, b)) return s;
+    s = count_once(p, b, st, sync);
+    if (s != NBL_ERROR_OUT_OF_MEMORY) return s;
+    // no room for more: as the first time, and so for these sizes from now on
+    clear_error();
+    p.list_pairs = 0.0;
+    p.list_more = 0;
+    p.list_stay = true;
     return count_once(p, b, st, sync);
 }
 
@@ -1382,6 +1410,8 @@ nbl_status nbl_plan_trim(nbl_plan *plan) {
     drop_count_graph(plan->p);
     plan->p.ws.release();
     plan->p.have_count = false;
+    plan->p.most_natoms = -1;  // what the device had no room for it may have now
+    plan->p.list_stay = false;
     return NBL_SUCCESS;
 }
 

@@ -181,6 +181,8 @@ struct Plan {
     // (the sizes: atoms, table, row range; groups of chained chunks to plan for)
     int64_t list_natoms = -1, list_table = -1, list_lo = 0, list_hi = 0, list_more = 0;
     double list_pairs = 0.0;
+    bool list_stay = false;  // no room for more than the density's estimate
+    int64_t most_natoms = -1, most_table = -1, most_lo = 0, most_hi = 0, list_most = 0;
     // Row range of nbl_set_atom_range (global atom indices, [lo, hi)).
     int64_t i_lo = 0;
     int64_t i_hi = INT64_MAX;

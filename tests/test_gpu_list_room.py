@@ -1,5 +1,7 @@
 """Room of the neighbour lists: what the plan keeps stays in proportion to the pairs
 a system can have, whatever its shape, and the lists are the oracle's."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -168,3 +170,47 @@ def test_batch_of_droplets_has_room(oracle, capacity):
     assert info.lists and not info.by_atoms
     assert info.list_bytes >= 4 * off[-1]
     b.close()
+
+
+@pytest.mark.parametrize("place", ["bulk", "droplet"])
+@pytest.mark.parametrize("failures", [0, 1, 2, 3, 4])
+def test_device_without_room_for_the_lists(oracle, place, failures):
+    """Workspace growths that fail leave fewer lists, and rows without one to the
+    thread-per-atom fill; what there was room for is kept for these sizes, so that
+    later calls neither release nor grow the workspace."""
+    import torch
+    from matscipy_neighbours import _matscipy_neighbours as ext
+    ext.lib.nbl_debug_inject.argtypes = [ctypes.c_int, ctypes.c_int64]
+    n = 24000
+    pos, cell = _bulk(n)
+    if place == "droplet":
+        cell = 8.0 * cell
+    pbc = np.array([False] * 3)
+    want = oracle.oracle_neighbour_list("ijdDS", cell, pos, 6.0, pbc)
+    plan = _plan()
+    from matscipy_neighbours import neighbour_list
+    call = lambda: neighbour_list("ijdDS", positions=pos, cell=cell, pbc=pbc, cutoff=6.0)
+    if place == "droplet":   # room for a gas of the same sizes: only the second count grows
+        neighbour_list("i", positions=8.0 * pos, cell=cell, pbc=pbc, cutoff=6.0)
+    try:
+        ext.check(ext.lib.nbl_debug_inject(1, failures))
+        try:
+            got = call()
+        except MemoryError:   # more failures than smaller layouts
+            assert failures > 1
+            return
+        assert_same_lists(got, want, "ijdDS")
+        ext.check(ext.lib.nbl_debug_inject(1, 0))
+        first = list_info(plan)
+        assert bool(first.short_of_room) == (failures > 0 and first.list_bytes < 4 * len(want[0]))
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        ext.check(ext.lib.nbl_debug_inject(1, 1))   # a growth would fail
+        for _ in range(3):
+            assert_same_lists(call(), want, "ijdDS")
+            info = list_info(plan)
+            assert info.list_bytes == first.list_bytes
+            assert info.workspace_bytes == first.workspace_bytes
+        assert torch.cuda.mem_get_info()[0] == free
+    finally:
+        ext.check(ext.lib.nbl_debug_inject(1, 0))
