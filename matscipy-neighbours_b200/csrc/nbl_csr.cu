@@ -13,8 +13,8 @@
 // major.  With m kept pairs a row has m (m - 1) triplets; triplet
 // q = a (m - 1) + c' of the row is (kept[a], kept[c' + (c' >= a)]).  Two
 // passes, one warp per row, with one read of the total in between: count m;
-// then list the kept pairs in shared memory and write the triplets
-// lane-parallel (consecutive lanes, consecutive triplets).  The
+// then list the kept pairs (in shared memory up to kRowKeep of them) and write
+// the triplets lane-parallel (consecutive lanes, consecutive triplets).  The
 // triplets of 5.4 M pairs of a 132,651-atom crystal, from the pair list: 247 us in
 // two calls that each counted and scanned, 116 so.
 #include <algorithm>
@@ -106,7 +106,14 @@ k_trip_count(const int32_t *__restrict__ first, int64_t nrows, const double *__r
     }
 }
 
-constexpr int kRowKeep = 128;  // kept pairs of a row listed in shared memory
+// Kept pairs of a row listed in shared memory.  A longer row takes the list from the
+// output: its last pair's partners are the other kept pairs in order, so that part of
+// ik is written first and read for the rest, eight rounds of loads before their
+// stores.  The call, for rows that keep some 130 of 2,000 pairs 220 us (3,000 rows;
+// 375 from a list of their own in device memory, 2,440 walking the row for every kept
+// pair), 400 of 500 590 (2,000 rows; 815, 1,170), 540 of 700 1,205 (2,000; 1,330),
+// 1,900 of 2,000 8.2 ms (300; 9.5).
+constexpr int kRowKeep = 512;
 
 __global__ void __launch_bounds__(kCsrThreads)
 k_trip_fill(const int32_t *__restrict__ first, int64_t nrows, const double *__restrict__ d,
@@ -122,19 +129,22 @@ k_trip_fill(const int32_t *__restrict__ first, int64_t nrows, const double *__re
         const int64_t b = first[r], e = first[r + 1], tb = toff[r];
         const int t = (int)(toff[r + 1] - tb);
         if (b < 0 || t == 0) continue;
-        int m = 0;
+        const int m1 = (int)__dsqrt_rn((double)t);  // t = m1 (m1 + 1)
+        const bool small = m1 < kRowKeep;
+        int32_t *list = small ? keep[warp] : ik + tb + (int64_t)m1 * m1;
+        int m = 0, last = 0;
         __syncwarp();
         for (int64_t p0 = b; p0 < e; p0 += 32) {
             const int64_t p = p0 + lane;
             const bool k = p < e && kept(d, cutoff, p);
             const unsigned bal = __ballot_sync(full, k);
             const int c = m + __popc(bal & lt);
-            if (k && c < kRowKeep) keep[warp][c] = (int32_t)p;
+            if (k && c < (small ? kRowKeep : m1)) list[c] = (int32_t)p;
+            if (bal) last = (int32_t)(p0 + 31 - __clz(bal));
             m += __popc(bal);
         }
         __syncwarp();
-        const int m1 = m - 1;
-        if (m <= kRowKeep) {
+        if (small) {
             for (int q = lane; q < t; q += 32) {
                 const int a = q / m1;
                 const int c1 = q - a * m1;
@@ -144,24 +154,29 @@ k_trip_fill(const int32_t *__restrict__ first, int64_t nrows, const double *__re
             }
             continue;
         }
-        // a longer row: its pairs are walked again for every kept one
-        int64_t out = tb;
-        for (int64_t p0 = b; p0 < e; p0 += 32) {
-            unsigned heads = __ballot_sync(full, p0 + lane < e && kept(d, cutoff, p0 + lane));
-            for (; heads; heads &= heads - 1u) {
-                const int64_t pa = p0 + __ffs(heads) - 1;
-                for (int64_t q0 = b; q0 < e; q0 += 32) {
-                    const int64_t q = q0 + lane;
-                    const bool k = q < e && q != pa && kept(d, cutoff, q);
-                    const unsigned bal = __ballot_sync(full, k);
-                    if (k) {
-                        __stcs(ij + out + __popc(bal & lt), (int32_t)pa);
-                        __stcs(ik + out + __popc(bal & lt), (int32_t)q);
-                    }
-                    out += __popc(bal);
-                }
+        const int32_t *from = ik + tb + (int64_t)m1 * m1;
+        const int body = t - m1;
+        for (int q0 = 0; q0 < body; q0 += 256) {
+            int va[8], vc[8];  // the loads before the stores, which may alias them
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int q = min(q0 + 32 * u + lane, body - 1);
+                const int a = q / m1;
+                const int c1 = q - a * m1;
+                const int c = c1 + (c1 >= a ? 1 : 0);
+                va[u] = from[a];
+                vc[u] = from[min(c, m1 - 1)];
+                if (c == m1) vc[u] = last;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int q = q0 + 32 * u + lane;
+                if (q >= body) break;
+                __stcs(ij + tb + q, va[u]);
+                __stcs(ik + tb + q, vc[u]);
             }
         }
+        for (int q = t - m1 + lane; q < t; q += 32) __stcs(ij + tb + q, last);
     }
 }
 
