@@ -626,7 +626,9 @@ __device__ __forceinline__ void lj_pair(const TraverseArgs &a, double dx, double
     f[3] += 0.5 * a.lj_eps4 * (s6 * s6 - s6);
 }
 
-// FP32 thresholds for one (atom, candidate) pair.
+// FP32 thresholds for one (atom, candidate) pair.  A pair cutoff that is not a number
+// gives thresholds that are none: no distance is below them, as in the exact test.
+__device__ __forceinline__ float narrower(float t, float rc) { return t >= rc ? rc : t; }
 template <int KIND>
 __device__ __forceinline__ void thresholds(const Hot &H, const TraverseArgs &a, float wi,
                                            float wj, float &lo, float &hi) {
@@ -635,14 +637,14 @@ __device__ __forceinline__ void thresholds(const Hot &H, const TraverseArgs &a, 
     if (KIND == kCutPerAtom) {
         const float cc = wi + wj;
         const float t = cc * cc;
-        lo = fminf(lo, t - H.band);
-        hi = fminf(hi, t + H.band);
+        lo = narrower(t - H.band, lo);
+        hi = narrower(t + H.band, hi);
     } else if (KIND == kCutPerType) {
         const int ti = __float_as_int(wi), tj = __float_as_int(wj);
         if (ti >= 0 && ti < H.ncut && tj >= 0 && tj < H.ncut) {
             const float t = a.pt32[H.pt_base + ti * H.ncut + tj];
-            lo = fminf(lo, t - H.band);
-            hi = fminf(hi, t + H.band);
+            lo = narrower(t - H.band, lo);
+            hi = narrower(t + H.band, hi);
         }
     }
 }
