@@ -185,29 +185,35 @@ __device__ __forceinline__ int list_stage_near(ListWarp<WIDE> &sm, const Travers
     return n;
 }
 
+// Per-type cutoffs: the squared cutoffs of one atom's type, and minus the one with
+// type tj (the widest for a type outside the table; a NaN stays one: neither sign bit
+// of the sums it enters is set).  One load a pair in the sweep: a million atoms with
+// cutoffs of 5, 3.2 and 3 take 1,500 us, with 5, 5 and 5 1,730; sweeping with the widest
+// and testing what that leaves pair by pair 2,030 and 2,110.
+struct TypeRow {
+    const float *at;
+    int n;
+};
+__device__ __forceinline__ TypeRow type_row(const TraverseArgs &a, const SysDev &S, float w) {
+    const int t = __float_as_int(w);
+    const bool in = t >= 0 && t < S.ncutoffs;
+    return TypeRow{a.pt32 + S.pt_base + (in ? t * S.ncutoffs : 0), in ? S.ncutoffs : 0};
+}
+__device__ __forceinline__ float type_cut(const TypeRow &row, int tj, float rc2) {
+    const float v = (unsigned)tj < (unsigned)row.n ? __ldg(row.at + tj) : rc2;
+    return v >= rc2 ? -rc2 : -v;
+}
+
 // Staged candidate k against atom il of the tile where the FP32 filter does not
-// decide: the pair's own threshold (per-type cutoffs), then the reference's
-// exact test.
+// decide: the reference's exact test.
 template <int KIND, bool WIDE>
 __device__ __noinline__ bool list_exact(const ListWarp<WIDE> &sm, const TraverseArgs &a,
-                                        const SysDev &S, float lo_rc, float hi_rc, float band,
-                                        int il, int k) {
+                                        const SysDev &S, int il, int k) {
     Hot H;
-    H.lo_rc = lo_rc;
-    H.hi_rc = hi_rc;
-    H.band = band;
     H.cutoff_sq = S.cutoff_sq;
     H.ncut = S.ncutoffs;
     H.pt_base = S.pt_base;
     const float4 c = sm.cand[k], p = sm.i32[il];
-    if (KIND == kCutPerType) {
-        const float dx = c.x - p.x, dy = c.y - p.y, dz = c.z - p.z;
-        const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-        float lo, hi;
-        thresholds<KIND>(H, a, p.w, c.w, lo, hi);
-        if (r2 < lo) return true;
-        if (!(r2 < hi)) return false;
-    }
     const int si = sm.isi[il];
     int sj, v;
     Entry<WIDE>::get(a.list_shift, sm.entry[k], sj, v);
@@ -413,8 +419,8 @@ k_count_list(const __grid_constant__ TraverseArgs a) {
         }
         const float2 nhi = make_float2(-hi_rc, -hi_rc), nlo = make_float2(-lo_rc, -lo_rc);
         const float2 minus1 = make_float2(-1.f, -1.f);
-        const bool sure_ok = KIND == kCutScalar ||
-                             (KIND == kCutPerAtom && !(*a.err & kNoteWideRadius));
+        const bool sure_ok = KIND != kCutPerAtom || !(*a.err & kNoteWideRadius);
+        const float rc2 = __double2float_rn(S.cutoff_sq);
         const float2 pband = make_float2(band, band), nband = make_float2(-band, -band);
         const int nvisit = S.nvisit;
         bool boxed = false;
@@ -463,6 +469,13 @@ k_count_list(const __grid_constant__ TraverseArgs a) {
                     // candidate inside the inner: the sign of r2 - threshold, shifted
                     // in (the comparison and the bit in one ALU operation)
                     unsigned near[4] = {0u, 0u, 0u, 0u}, sure[4] = {0u, 0u, 0u, 0u};
+                    TypeRow row[4];
+                    if (KIND == kCutPerType) {
+                        row[0] = type_row(a, S, p0.w);
+                        row[1] = type_row(a, S, p1.w);
+                        row[2] = type_row(a, S, p2.w);
+                        row[3] = type_row(a, S, p3.w);
+                    }
 #pragma unroll 2
                     for (int t = 0; t < blk; t++) {
                         const float4 c = mine[t];
@@ -490,6 +503,16 @@ k_count_list(const __grid_constant__ TraverseArgs a) {
                             ob = __fadd2_rn(eb, nband);
                             ia = __fadd2_rn(ea, pband);
                             ib = __fadd2_rn(eb, pband);
+                        } else if (KIND == kCutPerType) {
+                            const int tj = __float_as_int(c.w);
+                            const float2 ea = __fadd2_rn(ra, make_float2(type_cut(row[0], tj, rc2),
+                                                                         type_cut(row[1], tj, rc2)));
+                            const float2 eb = __fadd2_rn(rb, make_float2(type_cut(row[2], tj, rc2),
+                                                                         type_cut(row[3], tj, rc2)));
+                            oa = __fadd2_rn(ea, nband);
+                            ob = __fadd2_rn(eb, nband);
+                            ia = __fadd2_rn(ea, pband);
+                            ib = __fadd2_rn(eb, pband);
                         } else {
                             oa = __fadd2_rn(ra, nhi);
                             ob = __fadd2_rn(rb, nhi);
@@ -500,12 +523,10 @@ k_count_list(const __grid_constant__ TraverseArgs a) {
                         near[1] = __funnelshift_l(__float_as_uint(oa.y), near[1], 1);
                         near[2] = __funnelshift_l(__float_as_uint(ob.x), near[2], 1);
                         near[3] = __funnelshift_l(__float_as_uint(ob.y), near[3], 1);
-                        if (KIND != kCutPerType) {
-                            sure[0] = __funnelshift_l(__float_as_uint(ia.x), sure[0], 1);
-                            sure[1] = __funnelshift_l(__float_as_uint(ia.y), sure[1], 1);
-                            sure[2] = __funnelshift_l(__float_as_uint(ib.x), sure[2], 1);
-                            sure[3] = __funnelshift_l(__float_as_uint(ib.y), sure[3], 1);
-                        }
+                        sure[0] = __funnelshift_l(__float_as_uint(ia.x), sure[0], 1);
+                        sure[1] = __funnelshift_l(__float_as_uint(ia.y), sure[1], 1);
+                        sure[2] = __funnelshift_l(__float_as_uint(ib.x), sure[2], 1);
+                        sure[3] = __funnelshift_l(__float_as_uint(ib.y), sure[3], 1);
                     }
                     // first candidate of the block at the top bit; an atom is not its
                     // own neighbour
@@ -526,7 +547,7 @@ k_count_list(const __grid_constant__ TraverseArgs a) {
                         for (int g = 0; g < 4; g++)
                             for (unsigned open = near[g] ^ sure[g]; open; open &= open - 1u) {
                                 const unsigned low = open & (0u - open);
-                                if (list_exact<KIND, WIDE>(sm, a, S, lo_rc, hi_rc, band, g0 + g,
+                                if (list_exact<KIND, WIDE>(sm, a, S, g0 + g,
                                                            lane * blk + __clz(low)))
                                     sure[g] |= low;
                             }
