@@ -338,11 +338,12 @@ int64_t ListPlan::cap(const Batch &b, size_t s) const {
 
 // Whether the atoms are ordered by counting them into cells (cell_order) instead
 // of a radix sort of their cell keys: where the keys number the table's entries
-// (not Morton codes) and the table is within the size the automatic grid choice
-// allows, so that scanning it stays small beside the atoms.
+// (not Morton codes), the table is within the size the automatic grid choice allows,
+// so that scanning it stays small beside the atoms, and the cells are not crowded.
 static bool counted_cells(const Batch &b) {
     return b.grid != kGridMorton &&
-           b.table_size <= std::max<int64_t>(int64_t(1) << 20, 8 * b.natoms);
+           b.table_size <= std::max<int64_t>(int64_t(1) << 20, 8 * b.natoms) &&
+           b.natoms <= kRankAtoms * b.table_size;
 }
 
 // Carve the per-call buffers out of the plan's workspace, with lists of at most

@@ -110,6 +110,12 @@ constexpr int64_t kMarkAtoms = 131072;
 // Host positions of up to this many atoms are uploaded with the host tables: one
 // copy from pinned memory instead of that and one from pageable memory.
 constexpr int64_t kTablePositions = 2048;
+// Mean atoms per cell up to which the atoms are counted into cells and ranked there,
+// each by reading its cell's atoms; the radix sort above.  Binning to gather, ranked /
+// sorted: 2,000 atoms at 150 per cell 15 / 16 us, at 1,000 50 / 18; 20,000 at 150 / 300
+// / 1,000 16 / 23, 19 / 20, 60 / 19; 200,000 39 / 47, 63 / 40, 115 / 40; a million
+// 109 / 107, 150 / 104, 371 / 105.
+constexpr int64_t kRankAtoms = 192;
 // Atoms per occupied cell below which the count takes one thread per atom
 // (k_rows_count against k_count_list: 84 / 214 us at 2.3, 674 / 490 at 10).
 constexpr double kSparseAtoms = 4.0;

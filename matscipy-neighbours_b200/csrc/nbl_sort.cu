@@ -10,10 +10,12 @@
 // kernel counts them (and each atom's arrival in its cell); a scan gives the
 // slices, one kernel drops every atom into its slice in arrival order, and the
 // gather ranks an atom among its cell's by index, which restores the ascending
-// order.  The ranking reads every atom of a cell for every atom of it, 1/27 of
-// what the pair pass does with them, so no occupancy makes it dominate.  Against
-// two radix passes, init to gather: 13 -> 6 launches, 62 -> 36 us on the device for
-// a 200,000-atom gas, 33 -> 20 us for 10,007 atoms.
+// order.  The ranking reads every atom of a cell for every atom of it, as often as the
+// count of an isolated cell does and a 27th of what it does in a bulk; above kRankAtoms
+// atoms per cell on average the radix sort takes over (one crowded cell among many
+// stays with the ranking: 10,000 atoms there take 0.2 ms of it, the count 1 ms).
+// Against two radix passes, init to gather: 13 -> 6 launches, 62 -> 36 us on the
+// device for a 200,000-atom gas, 33 -> 20 us for 10,007 atoms.
 //
 // Scan: three-phase (tile reduce -> recursive scan of tile sums -> tile scan
 // with carry-in); no inter-block waiting, so no spin loops at all.

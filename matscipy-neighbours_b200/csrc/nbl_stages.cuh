@@ -103,9 +103,16 @@ __device__ __forceinline__ void gather_one(const GatherArgs &a, int64_t s) {
         if (a.skeys != nullptr) {  // the atom's rank in its cell, by index
             key = a.keys[at];
             seg = a.table[key];
-            int rank = 0;
+            int rank = 0, q = seg.x;
+            for (; q + 16 <= seg.y; q += 16) {  // a crowded cell: loads in flight
+                int v[16];
+#pragma unroll
+                for (int u = 0; u < 16; u++) v[u] = a.vals[q + u];
+#pragma unroll
+                for (int u = 0; u < 16; u++) rank += v[u] < at ? 1 : 0;
+            }
 #pragma unroll 4
-            for (int q = seg.x; q < seg.y; q++) rank += a.vals[q] < at ? 1 : 0;
+            for (; q < seg.y; q++) rank += a.vals[q] < at ? 1 : 0;
             s = seg.x + rank;
             a.skeys[s] = key;
         } else {
