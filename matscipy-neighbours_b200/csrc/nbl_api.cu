@@ -634,16 +634,43 @@ static bool sparse_grid(const Plan &p, const Batch &b) {
     return (double)b.natoms < kSparseAtoms * cells;
 }
 
-// Whether the force pass takes one thread per atom (k_atoms_lj) instead of the
-// work items (k_count_list): for cutoffs by atom or type, and on sparse grids.
-// Measured (us, by items / by atoms): 200,001 atoms at 1 / 2.9 / 3.3 / 13 per cell
-// 214 / 64, 152 / 117, 145 / 121, 198 / 249; 20,001 atoms at 0.5 / 1.4 / 2.4 / 13
-// 31 / 25, 31 / 47, 25 / 53, 50 / 129; 7,483 at 11 24 / 101.
-static bool lj_by_atoms(const Batch &b) {
-    if (b.sys.empty() || b.sys[0].cutoff_kind != kCutScalar) return true;
+// Sizes that a note of occupied cells is for.
+static uint32_t occupied_tag(const Batch &b) {
+    return (uint32_t)b.natoms * 2654435761u ^ (uint32_t)b.table_size;
+}
+
+// Atoms per occupied cell below which the force pass takes one thread per atom
+// (k_atoms_lj) instead of the work items (k_count_list).  Measured, us by atoms / by
+// items, where the two cross: 7,483 atoms at 1.2 36 / 20; 20,001 at 1.2 / 1.6 36 / 36,
+// 51 / 34; 65,000 at 2.3 / 3.1 65 / 71, 75 / 69; 200,001 at 5.1 / 6.1 177 / 180,
+// 195 / 181; a million at 6.0 / 8.0 / 10 699 / 825, 807 / 796, 924 / 845, as a droplet
+// at 7.5 698 / 807.  (The more atoms, the less the length of one thread's walk matters.)
+static double lj_line(int64_t natoms) {
+    return std::max(2.0 * (std::log((double)std::max<int64_t>(natoms, 1)) - 9.4), 0.0);
+}
+
+// Which of the two the force pass takes for batch b: p.sparse (also for cutoffs by atom
+// or type and plain FP64 tests), and the line to give the kernels: 0, or, where only the
+// device can tell, lj_line; both are launched then, and the one that the occupied cells
+// rule out returns at once (3 us).  All cells, empty ones too, tell that a grid is dense;
+// what the last force pass of these sizes found occupied (it writes that to the plan's
+// pinned words, nothing waits for it) tells the rest.  Without it a droplet in a wide box
+// looked sparse: 7,483 atoms 228 us a call, 135 now.
+static float choose_lj(Plan &p, const Batch &b) {
+    p.sparse = !b.fp32 || b.sys.empty() || b.sys[0].cutoff_kind != kCutScalar;
+    if (p.sparse) return 0.f;
+    const double line = lj_line(b.natoms);
     double cells = 0.0;
     for (int64_t n : b.ncells) cells += (double)n;
-    return (double)b.natoms < (b.natoms <= 65536 ? 1.0 : 4.0) * cells;
+    if ((double)b.natoms >= line * cells) return 0.f;
+    const unsigned long long note = *reinterpret_cast<volatile unsigned long long *>(
+        p.host_small + kOccupiedWord);
+    const double occupied = (double)(uint32_t)note;
+    if (occupied > 0.0 && (uint32_t)(note >> 32) == occupied_tag(b)) {
+        p.sparse = (double)b.natoms < line * occupied;
+        return 0.f;
+    }
+    return (float)line;
 }
 
 // Size the workspace for a batch and copy its inputs and host tables in.
@@ -653,7 +680,7 @@ nbl_status upload_batch(Plan &p, const Batch &b, cudaStream_t st, CountUse use) 
     p.forces = use == kUseForces;
     p.rows = p.forces || (use == kUseLists && p.atom_threads == 0 && p.max_run == 0);
     p.sparse = p.rows && (!b.fp32 || sparse_grid(p, b));
-    if (p.forces) p.sparse = !b.fp32 || lj_by_atoms(b);
+    if (p.forces) p.lj_line = choose_lj(p, b);
     p.cand_atom = candidates_per_atom(b);
     nbl_status s = layout_workspace(p, b);
     if (s != NBL_SUCCESS) return s;
@@ -1346,7 +1373,8 @@ nbl_status plan_init(Plan &p, int device_id) {
     DeviceGuard g(dev);
     NBL_CUDA(cudaDeviceGetAttribute(&p.num_sms, cudaDevAttrMultiProcessorCount, dev),
              "device query");
-    NBL_CUDA(cudaMallocHost(&p.host_small, sizeof(int64_t) * 4), "pinned");
+    NBL_CUDA(cudaMallocHost(&p.host_small, sizeof(int64_t) * 8), "pinned");
+    p.host_small[kOccupiedWord] = 0;
     NBL_CUDA(cudaEventCreateWithFlags(&p.stage_done, cudaEventDisableTiming), "event");
     return NBL_SUCCESS;
 }
@@ -1695,9 +1723,13 @@ nbl_status nbl_lj_forces(nbl_plan *plan, const nbl_request *req, double epsilon,
     ta.lj_eps24 = 24.0 * epsilon;
     ta.lj_sig2 = sigma * sigma;
     ta.ticket_ready = 1;  // k_init cleared the ticket
-    NBL_CUDA(p.sparse ? launch_lj_atoms(p.batch_kind, ta, cs)
-                      : launch_lj_list(p.cand_atom > kCullCand, ta, p.num_sms, cs),
-             "force pass");
+    ta.lj_line = p.lj_line;
+    ta.occupied_note = reinterpret_cast<unsigned long long *>(p.host_small + kOccupiedWord);
+    ta.occupied_tag = occupied_tag(b);
+    if (p.sparse || p.lj_line > 0.f)
+        NBL_CUDA(launch_lj_atoms(p.batch_kind, ta, cs), "force pass");
+    if (!p.sparse)
+        NBL_CUDA(launch_lj_list(p.cand_atom > kCullCand, ta, p.num_sms, cs), "force pass");
     NBL_CUDA(launch_lj_energy(p.bufs.lj_part, b.natoms, p.bufs.lj_part + b.natoms, energy,
                               cs),
              "energy");

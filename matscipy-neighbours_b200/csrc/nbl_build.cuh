@@ -107,6 +107,10 @@ struct TraverseArgs {
     double *lj_force;
     double *lj_energy;
     double lj_eps4, lj_eps24, lj_sig2;
+    float lj_line;            // > 0: atoms per occupied cell below which k_atoms_lj does the
+                              // work, else k_count_list (both launched); 0: the one launched
+    unsigned long long *occupied_note;  // pinned host word: occupied cells, tag above
+    uint32_t occupied_tag;
     int *err;
     // Rows produced: only atoms whose global index lies in [i_lo, i_hi) act
     // as i; every atom stays a candidate j.  Rows outside keep count 0.

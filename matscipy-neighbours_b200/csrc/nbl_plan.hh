@@ -135,6 +135,8 @@ struct CountKey {
     bool operator==(const CountKey &o) const { return std::memcmp(this, &o, sizeof(*this)) == 0; }
 };
 
+constexpr int kOccupiedWord = 4;  // of Plan::host_small
+
 // What a batch is uploaded for.
 enum CountUse { kUseLists, kUseOneLaunch, kUseForces };
 
@@ -181,6 +183,7 @@ struct Plan {
     bool rows = false;
     double cand_atom = 0.0;   // atoms of the cells that an atom visits, on average
     bool forces = false;      // a force pass: no lists planned
+    float lj_line = 0.f;      // its choice left to the device (choose_lj)
     bool sparse = false;      // with one thread per atom in the count
     bool spare_ticket = false;  // a cleared work-item ticket is left for one fill
     bool lists_short = true;  // some row may have no list (kErrNoList)
@@ -201,7 +204,9 @@ struct Plan {
     bool count_pending = false;   // a force pass left no counts: made on demand
     int64_t npairs = 0;
     int quantities = 0;
-    int64_t *host_small = nullptr;  // pinned: [0] pair count, [1] flags
+    // pinned: [0] pair count, [1] flags, [kOccupiedWord] occupied cells of the last force
+    // pass (low half) and the sizes they belong to
+    int64_t *host_small = nullptr;
     void *host_stage = nullptr;     // pinned staging of the small host tables
     size_t host_stage_bytes = 0;
     void *host_out = nullptr;       // pinned landing area of small host fills

@@ -287,6 +287,8 @@ template <int KIND>
 __global__ void __launch_bounds__(kAtomThreads)
 k_atoms_lj(const __grid_constant__ TraverseArgs a) {
     const int64_t si = (int64_t)blockIdx.x * kAtomThreads + threadIdx.x;
+    lj_note(a);
+    if (a.lj_line > 0.f && !lj_sparse(a)) return;
     if (si < a.natoms) atom_lj<KIND>(a, si);
 }
 

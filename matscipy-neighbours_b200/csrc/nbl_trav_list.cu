@@ -377,6 +377,10 @@ k_count_list(const __grid_constant__ TraverseArgs a) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     ListWarp<WIDE> &sm = reinterpret_cast<ListWarp<WIDE> *>(dyn_smem)[warp];
     double (*acc)[4] = acc_all[LJ ? warp : 0];
+    if (LJ) {
+        lj_note(a);
+        if (a.lj_line > 0.f && lj_sparse(a)) return;
+    }
     const int nitems = *a.n_items;
     ItemLoop L(a, (int)blockIdx.x * kListWarps + warp, nitems, lane, false);
     while (L.it < nitems) {

@@ -611,6 +611,18 @@ __device__ __forceinline__ float3 run_frame32(const SysDev &S, int t) {
                        __double2float_rn(o[2]));
 }
 
+// The occupied cells, for the host's choice at a later force pass.
+__device__ __forceinline__ void lj_note(const TraverseArgs &a) {
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        *reinterpret_cast<volatile unsigned long long *>(a.occupied_note) =
+            (unsigned long long)a.occupied_tag << 32 | (unsigned)*a.n_home;
+}
+
+// Whether the occupied cells hold few enough atoms for the force pass by atoms.
+__device__ __forceinline__ bool lj_sparse(const TraverseArgs &a) {
+    return (float)a.natoms < a.lj_line * (float)*a.n_home;
+}
+
 // One pair's force on atom i and energy share (lj_langevin_gpu.cu:59-74): U =
 // 4 eps ((sigma/r)^12 - (sigma/r)^6) cut at the list's cutoff, F_i = -24 eps s6
 // (2 s6 - 1) D / r^2, half of U per directed pair.
