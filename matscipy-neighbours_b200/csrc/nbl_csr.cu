@@ -35,6 +35,21 @@ constexpr int kCsrThreads = 256;
 constexpr int kCsrWarps = kCsrThreads / 32;
 constexpr int kMaxKept = 46340;  // m (m - 1) stays below 2^31
 
+// Kept pairs of a row that a warp lists in shared memory.  A longer row is written by
+// a CTA, a warp per first pair (no division), from all of its shared memory, or, beyond
+// that, from the output: the last pair's partners are the other kept pairs in order, so
+// that part of ik is written first and read for the rest.  The call, for rows that keep
+// 140 of 150 pairs 800 us (20,000 rows; 960 from a list of their own in device memory,
+// 1,000 with 128 here), 400 of 500 620 (2,000 rows; 800, and 1,170 walking the row for
+// every kept pair), 500 of 600 1,230 (2,000; 1,140, 1,720), 540 of 700 1,110 (2,000;
+// 1,315, 2,220), 1,900 of 2,000 2.1 ms (300; 9.5, 21.4), 2,400 of 2,600 5.0 (300; 15.1,
+// 42.9).
+constexpr int kRowKeep = 256;
+
+// Bits that the count leaves beside the total.
+constexpr int kTripMany = 1;  // a row keeps more than kMaxKept pairs
+constexpr int kTripLong = 2;  // a row keeps more than kRowKeep
+
 __global__ void k_seed_init(int64_t n, int32_t v, int32_t *__restrict__ seed) {
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k <= n) seed[k] = v;
@@ -83,7 +98,7 @@ __device__ __forceinline__ bool kept(const double *d, double cutoff, int64_t p) 
 // before the first one with pairs) hold none.
 __global__ void __launch_bounds__(kCsrThreads)
 k_trip_count(const int32_t *__restrict__ first, int64_t nrows, const double *__restrict__ d,
-             double cutoff, int32_t *__restrict__ tcount, unsigned long long *__restrict__ err) {
+             double cutoff, int32_t *__restrict__ tcount, int *__restrict__ flags) {
     const int lane = threadIdx.x & 31;
     const int64_t gw = ((int64_t)blockIdx.x * kCsrThreads + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * kCsrThreads) >> 5;
@@ -98,28 +113,23 @@ k_trip_count(const int32_t *__restrict__ first, int64_t nrows, const double *__r
         }
         if (lane == 0) {
             if (m > kMaxKept) {
-                atomicOr(err, 1ull);
+                atomicOr(flags, kTripMany);
                 m = 0;
             }
+            if (m > kRowKeep) atomicOr(flags, kTripLong);
             tcount[r] = m * (m - 1) > 0 ? m * (m - 1) : 0;
         }
     }
 }
 
-// Kept pairs of a row listed in shared memory.  A longer row takes the list from the
-// output: its last pair's partners are the other kept pairs in order, so that part of
-// ik is written first and read for the rest, eight rounds of loads before their
-// stores.  The call, for rows that keep some 130 of 2,000 pairs 220 us (3,000 rows;
-// 375 from a list of their own in device memory, 2,440 walking the row for every kept
-// pair), 400 of 500 590 (2,000 rows; 815, 1,170), 540 of 700 1,205 (2,000; 1,330),
-// 1,900 of 2,000 8.2 ms (300; 9.5).
-constexpr int kRowKeep = 512;
-
-__global__ void __launch_bounds__(kCsrThreads)
+// (Eight CTAs per SM: with 61 registers instead of 32 the short rows of 5.4 M pairs took
+// 39 us, 33 so.)
+__global__ void __launch_bounds__(kCsrThreads, 8)
 k_trip_fill(const int32_t *__restrict__ first, int64_t nrows, const double *__restrict__ d,
-            double cutoff, const int64_t *__restrict__ toff, int32_t *__restrict__ ij,
-            int32_t *__restrict__ ik) {
+            double cutoff, const int64_t *__restrict__ toff, const int *__restrict__ flags,
+            int32_t *__restrict__ ij, int32_t *__restrict__ ik) {
     __shared__ int32_t keep[kCsrWarps][kRowKeep];
+    __shared__ int32_t last;
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t gw = ((int64_t)blockIdx.x * kCsrThreads + threadIdx.x) >> 5;
@@ -128,63 +138,80 @@ k_trip_fill(const int32_t *__restrict__ first, int64_t nrows, const double *__re
     for (int64_t r = gw; r < nrows; r += nw) {
         const int64_t b = first[r], e = first[r + 1], tb = toff[r];
         const int t = (int)(toff[r + 1] - tb);
-        if (b < 0 || t == 0) continue;
-        const int m1 = (int)__dsqrt_rn((double)t);  // t = m1 (m1 + 1)
-        const bool small = m1 < kRowKeep;
-        int32_t *list = small ? keep[warp] : ik + tb + (int64_t)m1 * m1;
-        int m = 0, last = 0;
+        if (b < 0 || t == 0 || t > kRowKeep * (kRowKeep - 1)) continue;  // (below)
+        int m = 0;
         __syncwarp();
         for (int64_t p0 = b; p0 < e; p0 += 32) {
             const int64_t p = p0 + lane;
             const bool k = p < e && kept(d, cutoff, p);
             const unsigned bal = __ballot_sync(full, k);
             const int c = m + __popc(bal & lt);
-            if (k && c < (small ? kRowKeep : m1)) list[c] = (int32_t)p;
-            if (bal) last = (int32_t)(p0 + 31 - __clz(bal));
+            if (k && c < kRowKeep) keep[warp][c] = (int32_t)p;
             m += __popc(bal);
         }
         __syncwarp();
-        if (small) {
-            for (int q = lane; q < t; q += 32) {
-                const int a = q / m1;
-                const int c1 = q - a * m1;
-                const int c = c1 + (c1 >= a ? 1 : 0);
-                __stcs(ij + tb + q, keep[warp][a]);
-                __stcs(ik + tb + q, keep[warp][c]);
-            }
-            continue;
+        const int m1 = m - 1;
+        for (int q = lane; q < t; q += 32) {
+            const int a = q / m1;
+            const int c1 = q - a * m1;
+            const int c = c1 + (c1 >= a ? 1 : 0);
+            __stcs(ij + tb + q, keep[warp][a]);
+            __stcs(ik + tb + q, keep[warp][c]);
         }
-        const int32_t *from = ik + tb + (int64_t)m1 * m1;
-        const int body = t - m1;
-        for (int q0 = 0; q0 < body; q0 += 256) {
-            int va[8], vc[8];  // the loads before the stores, which may alias them
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const int q = min(q0 + 32 * u + lane, body - 1);
-                const int a = q / m1;
-                const int c1 = q - a * m1;
-                const int c = c1 + (c1 >= a ? 1 : 0);
-                va[u] = from[a];
-                vc[u] = from[min(c, m1 - 1)];
-                if (c == m1) vc[u] = last;
-            }
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const int q = q0 + 32 * u + lane;
-                if (q >= body) break;
-                __stcs(ij + tb + q, va[u]);
-                __stcs(ik + tb + q, vc[u]);
+    }
+    if (!(*flags & kTripLong)) return;
+    // --- long rows, one per CTA ---------------------------------------------------
+    int32_t *all = &keep[0][0];
+    __syncthreads();
+    for (int64_t r = blockIdx.x; r < nrows; r += gridDim.x) {
+        const int64_t b = first[r], tb = toff[r];
+        const int t = (int)(toff[r + 1] - tb);
+        if (b < 0 || t <= kRowKeep * (kRowKeep - 1)) continue;  // (the same for all threads)
+        const int m1 = (int)__dsqrt_rn((double)t);  // the kept pairs but one: t = m1 (m1 + 1)
+        const bool fits = m1 < kCsrWarps * kRowKeep;
+        int32_t *list = ik + tb + (t - m1);         // else: the kept pairs but the last
+        if (warp == 0) {
+            const int64_t e = first[r + 1];
+            int m = 0;
+            for (int64_t p0 = b; p0 < e; p0 += 32) {
+                const int64_t p = p0 + lane;
+                const bool k = p < e && kept(d, cutoff, p);
+                const unsigned bal = __ballot_sync(full, k);
+                const int c = m + __popc(bal & lt);
+                if (k && fits && c <= m1) all[c] = (int32_t)p;
+                if (k && !fits && c < m1) list[c] = (int32_t)p;
+                if (k && c == m1) last = (int32_t)p;
+                m += __popc(bal);
             }
         }
-        for (int q = t - m1 + lane; q < t; q += 32) __stcs(ij + tb + q, last);
+        __syncthreads();
+        for (int a = warp; a <= m1; a += kCsrWarps) {  // a warp per first pair
+            int32_t *oj = ij + tb + (int64_t)a * m1, *ok = ik + tb + (int64_t)a * m1;
+            if (fits) {
+                const int va = all[a];
+                for (int c = lane; c < m1; c += 32) {
+                    __stcs(oj + c, va);
+                    __stcs(ok + c, all[c + (c >= a ? 1 : 0)]);
+                }
+            } else {
+                const int va = a < m1 ? list[a] : last;
+                for (int c = lane; c < m1; c += 32) {
+                    const int k = c + (c >= a ? 1 : 0);
+                    __stcs(oj + c, va);
+                    if (a < m1) __stcs(ok + c, k < m1 ? list[k] : last);
+                }
+            }
+        }
+        __syncthreads();
     }
 }
 
-int trip_grid(int64_t nrows, int dev) {
+// CTAs: one per `rows` rows, at most eight per SM.
+int trip_grid(int64_t nrows, int rows, int dev) {
     int nsm = 148;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     return (int)std::max<int64_t>(
-        1, std::min<int64_t>((nrows + kCsrWarps - 1) / kCsrWarps, (int64_t)nsm * 8));
+        1, std::min<int64_t>((nrows + rows - 1) / rows, (int64_t)nsm * 8));
 }
 
 }  // namespace
@@ -244,7 +271,6 @@ extern "C" NBL_API nbl_status nbl_triplet_count(int64_t nfirst, const int32_t *f
         bytes += (b + 255) & ~size_t(255);
         return o;
     };
-    const size_t o_tick = add(sizeof(int));
     const size_t o_t = add(sizeof(int32_t) * nrows);
     const size_t o_s = add(sizeof(int64_t) * scan_scratch_elems(nrows + 1));
     {
@@ -252,23 +278,22 @@ extern "C" NBL_API nbl_status nbl_triplet_count(int64_t nfirst, const int32_t *f
         CSR_CUDA(scratch_pool(dev, &pool), "triplet scratch pool");
         CSR_CUDA(cudaMallocFromPoolAsync((void **)&scratch, bytes, pool, st), "triplet scratch");
         int32_t *tcount = reinterpret_cast<int32_t *>(scratch + o_t);
-        // the flag behind the total, so that one copy reads both
-        unsigned long long *err = reinterpret_cast<unsigned long long *>(row_offsets + nfirst);
-        CSR_CUDA(cudaMemsetAsync(err, 0, sizeof(*err), st), "memset");
-        CSR_CUDA(cudaMemsetAsync(scratch + o_tick, 0, sizeof(int), st), "memset");
-        k_trip_count<<<trip_grid(nrows, dev), kCsrThreads, 0, st>>>(first_i, nrows, absdist,
-                                                                    cutoff, tcount, err);
+        // behind the total, so that one copy reads both: the scan's ticket, the flags
+        int *word = reinterpret_cast<int *>(row_offsets + nfirst);
+        CSR_CUDA(cudaMemsetAsync(word, 0, sizeof(int64_t), st), "memset");
+        k_trip_count<<<trip_grid(nrows, kCsrWarps, dev), kCsrThreads, 0, st>>>(first_i, nrows, absdist,
+                                                                    cutoff, tcount, word + 1);
         count_launch();
         CSR_CUDA(cudaGetLastError(), "triplet count");
         CSR_CUDA(exclusive_scan_i32_i64(tcount, nrows, row_offsets,
                                         reinterpret_cast<int64_t *>(scratch + o_s), st,
-                                        reinterpret_cast<int *>(scratch + o_tick)),
+                                        word),
                  "scan");
         CSR_CUDA(cudaMemcpyAsync(host, row_offsets + nrows, 2 * sizeof(int64_t),
                                  cudaMemcpyDeviceToHost, st),
                  "read count");
         CSR_CUDA(cudaStreamSynchronize(st), "triplet count");
-        if (host[1]) {
+        if ((host[1] >> 32) & kTripMany) {
             status = set_error(NBL_ERROR_INVALID_ARGUMENT,
                                "triplet_list: a row keeps more than %d pairs", kMaxKept);
             goto done;
@@ -289,8 +314,10 @@ extern "C" NBL_API nbl_status nbl_triplet_fill(int64_t nfirst, const int32_t *fi
     if (nfirst < 2) return NBL_SUCCESS;
     int dev = 0;
     cudaGetDevice(&dev);
-    k_trip_fill<<<trip_grid(nfirst - 1, dev), kCsrThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        first_i, nfirst - 1, absdist, cutoff, row_offsets, ij, ik);
+    k_trip_fill<<<trip_grid(nfirst - 1, 1, dev), kCsrThreads, 0,
+                  static_cast<cudaStream_t>(stream)>>>(
+        first_i, nfirst - 1, absdist, cutoff, row_offsets,
+        reinterpret_cast<const int *>(row_offsets + nfirst) + 1, ij, ik);
     count_launch();
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? NBL_SUCCESS : cuda_status(e, "triplet fill");

@@ -1,12 +1,14 @@
-"""Triplets of rows that keep more pairs than the shared-memory list holds (512, two
-windows of 256): the host's list, and no cliff in time at that length."""
+"""Triplets of rows that keep more pairs than a warp's shared-memory list holds (256: a
+CTA takes over, up to 2,048 in its shared memory): the host's list, and no cliff in time
+where a row grows past the list."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("lengths", [[255, 256, 257], [511, 512, 513, 7], [640, 0, 900], [1300]])
+@pytest.mark.parametrize("lengths", [[255, 256, 257], [511, 512, 513, 7], [640, 0, 900], [1300],
+                                     [2047, 2048], [2049, 3], [2500]])
 @pytest.mark.parametrize("keep", [None, 0.15, 0.97])
 def test_long_rows(lengths, keep):
     import torch
