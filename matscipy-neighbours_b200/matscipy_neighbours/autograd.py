@@ -58,14 +58,16 @@ def _function():
                                     ctypes.c_void_p(pos.data_ptr()) if nat else None, True,
                                     rc, per_atom, per_type_sq, ncut, types, dev.index)
             n = ctypes.c_int64()
-            with torch.cuda.device(dev):
+
+            def count():
                 _ext.check(_ext.lib.nbl_count(plan, ctypes.byref(req), sp, ctypes.byref(n)))
+                return int(n.value)
+
+            with torch.cuda.device(dev):
+                bufs = _ext.with_room(plan, torch.OutOfMemoryError, count,
+                                      lambda P: _ext._device_outputs(torch, "ijDdS", P, dev))
+                i, j, D, d, S = (bufs[ch] for ch in "ijDdS")
                 P = int(n.value)
-                i = torch.empty(P, dtype=torch.int32, device=dev)
-                j = torch.empty(P, dtype=torch.int32, device=dev)
-                D = torch.empty((P, 3), dtype=torch.float64, device=dev)
-                d = torch.empty(P, dtype=torch.float64, device=dev)
-                S = torch.empty((P, 3), dtype=torch.int32, device=dev)
                 off = None  # (the default backward reads no row offsets)
                 if deterministic:
                     off = torch.empty(nat + 1, dtype=torch.int64, device=dev)
