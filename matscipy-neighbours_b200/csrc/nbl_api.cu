@@ -580,10 +580,12 @@ static double candidates_per_atom(const Batch &b) {
     return cand / (double)std::max<int64_t>(b.natoms, 1);
 }
 
-// Candidates per atom above which the list count drops those outside the
-// tile's bounding box before staging: two full tables.  Measured with and
-// without: 1,548 / 2,411 us at about 3,000, 527 / 490 us at 300.
-constexpr double kCullCand = 832.0;
+// Candidates per atom above which the list count drops those outside the tile's
+// bounding box before staging: one full table.  Measured with and without, us: a
+// million atoms of a metal at 300 527 / 490; uniform, 400,000 atoms at 330 / 549 / 781
+// / 1,575 225 / 222, 278 / 346, 392 / 439, 677 / 845; 20,000 at 312 / 540 / 1,055
+// 35 / 38, 39 / 57, 66 / 78; 4,096 small systems at about 3,000 1,548 / 2,411.
+constexpr double kCullCand = 416.0;
 
 // Atoms per work item (the cell-occupancy tile) for batch b: the launch
 // configuration's, or by default chosen from the atom count.  A small system
