@@ -102,13 +102,17 @@ struct Workspace {
 constexpr int kAutoWaves = 2;
 
 // Atoms above which the row of every 128th output slot is marked after the scan
-// (k_row_marks), if the pair count is known from an earlier count of the same
-// sizes (the marks' table has its size from there); below it the fill's warps search the row offsets.  Measured with and
-// without, fill + marks: 1,048,576 atoms 657 against 699 us, 200,000 27 against
-// 27, 132,651 76 against 76, 1,000 16 against 13.
+// (k_row_marks); below it, and beyond the marks' table, which has room for as many
+// pairs as the lists, the fill's warps search the row offsets.  Measured, fill and marks
+// with / without, us, uniform gases: a million atoms at 10 / 2 / 0.5 per cell 704 / 713,
+// 183 / 182, 74 / 73; 200,000 130 / 133, 37 / 38, 22 / 20; 131,072 81 / 86, 29 / 29,
+// 16 / 15; 30,000 30 / 30, 11 / 10, 11 / 10: a launch for little, paid back by long
+// lists.
 constexpr int64_t kMarkAtoms = 131072;
 // Host positions of up to this many atoms are uploaded with the host tables: one
-// copy from pinned memory instead of that and one from pageable memory.
+// copy from pinned memory instead of that and one from pageable memory.  The call, with
+// the tables / on their own: 1,000 atoms 115 / 117 us, 2,000 126 / 134, 16,000 182 /
+// 190, 32,000 250 / 233; the line keeps the pinned staging below 100 KB.
 constexpr int64_t kTablePositions = 2048;
 // Mean atoms per cell up to which the atoms are counted into cells and ranked there,
 // each by reading its cell's atoms; the radix sort above.  Binning to gather, ranked /
@@ -116,8 +120,11 @@ constexpr int64_t kTablePositions = 2048;
 // / 1,000 16 / 23, 19 / 20, 60 / 19; 200,000 39 / 47, 63 / 40, 115 / 40; a million
 // 109 / 107, 150 / 104, 371 / 105.
 constexpr int64_t kRankAtoms = 192;
-// Atoms per occupied cell below which the count takes one thread per atom
-// (k_rows_count against k_count_list: 84 / 214 us at 2.3, 674 / 490 at 10).
+// Atoms per occupied cell below which the count takes one thread per atom.  Measured,
+// k_rows_count / k_count_list, us: 20,000 atoms at 2.2 / 3.1 / 4.1 per occupied cell
+// 20 / 26, 21 / 25, 29 / 28; 60,000 at 2.3 / 3.2 / 3.9 41 / 54, 53 / 47, 52 / 46;
+// 200,000 at 3.1 / 4.0 / 5.1 99 / 129, 109 / 121, 125 / 113; a million at 4.1 / 6.0 /
+// 8.0 392 / 553, 470 / 490, 556 / 469.
 constexpr double kSparseAtoms = 4.0;
 
 // Everything that shapes the count phase's launches on a plan: when two

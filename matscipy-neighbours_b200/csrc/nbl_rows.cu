@@ -42,8 +42,12 @@ namespace nbl {
 namespace {
 
 constexpr int kRowThreads = 128;
+// Lanes per atom of a small system, and up to how many atoms (one thread per atom
+// leaves most of the chip idle there).  Count with eight lanes / one, us, at 0.5 and 2
+// atoms per cell: 2,000 atoms 9 / 26, 10 / 34; 16,000 15 / 27, 18 / 36; 32,000 22 / 29,
+// 28 / 38; 48,000 30 / 31, 37 / 41; 64,000 38 / 30, 46 / 43.
 constexpr long long kSplitAtoms = 32768;
-constexpr int kSplit = 8;      // lanes per atom of small systems
+constexpr int kSplit = 8;
 constexpr int kSplitBuf = 16;  // list entries a lane of those buffers
 
 // Appends to a row's list: entries gather in one group's registers and leave
