@@ -948,9 +948,9 @@ static nbl_status enqueue_count_pass(Plan &p, bool ticket_ready, cudaStream_t st
             NBL_CUDA(launch_count_list(p.batch_kind, p.cand_atom > kCullCand, tc, p.num_sms, st),
                      "count pass");
         else
-        NBL_CUDA(launch_traverse(kModeCount, p.batch_fp32, p.batch_kind, tc, p.trav_grid, st,
-                                 p.count_shape),
-                 "count pass");
+            NBL_CUDA(launch_traverse(kModeCount, p.batch_fp32, p.batch_kind, tc, p.trav_grid,
+                                     st, p.count_shape),
+                     "count pass");
     }
     {
         StageRange r("nbl.scan");

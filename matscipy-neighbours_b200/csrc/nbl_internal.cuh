@@ -12,8 +12,10 @@
 //   pos64[N]  double4   cell-sorted bin-relative position (x, y, z), the FP64
 //                       operands, and in the bits of w the global atom index
 //                       (low word) and the packed image index (high word)
-//   pos32[N]  float4    the same position rounded to FP32 (x, y, z) and the
-//                       per-atom radius (FP32) or the type id (int bits) (w)
+//   pos32[N]  float4    the same position in FP32 (x, y, z), for the counts by atoms
+//                       (nbl_rows.cu) relative to the first cell of the atom's row
+//                       along x, and the per-atom radius (FP32) or the type id (int
+//                       bits) (w)
 //   aux[N]    int4      (global atom index, q0, q1, q2): q is the atom's
 //                       periodic image index (periodic axes) or the
 //                       reference's shift quirk (non-periodic axes)

@@ -87,7 +87,7 @@ struct Bufs {
     int32_t *inv = nullptr;
     int32_t *row_of = nullptr;
     ListPlan list_plan;
-    double *lj_part = nullptr;     // force sink: per-atom energies, then block sums
+    double *lj_part = nullptr;     // force pass: per-atom energies, then block sums
 };
 
 struct Workspace {

@@ -399,8 +399,8 @@ __device__ __forceinline__ bool list_entry(const TraverseArgs &a, long long base
     return !checked_fail(sj < 0 || sj >= a.natoms, a.err);
 }
 
-// Image shift of visit v from home cell hc, packed or (false) not packable.
-__device__ __forceinline__ bool visit_image(const TraverseArgs &a, const SysDev &S, const int4 &hc,
+// Image shift of visit v from home cell hc.
+__device__ __forceinline__ void visit_image(const TraverseArgs &a, const SysDev &S, const int4 &hc,
                                             int v, int m[3]) {
     int d[3];
     float unused[3];
@@ -412,7 +412,6 @@ __device__ __forceinline__ bool visit_image(const TraverseArgs &a, const SysDev 
         m[k] = x < 0 ? (x >= -n ? -1 : floor_div(x, n))
                      : x >= n ? (x < 2 * n ? 1 : floor_div(x, n)) : 0;
     }
-    return true;
 }
 
 // S of one pair whose image indices do not pack, from the full records.

@@ -558,7 +558,7 @@ k_count_list(const __grid_constant__ TraverseArgs a) {
                         __syncwarp();
                     }
                     list_pair<WIDE, LJ>(sm, acc, a, S, sure[0], sure[1], g0, blk, lane);
-                    if (g0 + 2 < ni) 
+                    if (g0 + 2 < ni)
                         list_pair<WIDE, LJ>(sm, acc, a, S, sure[2], sure[3], g0 + 2, blk, lane);
                 }
             }
