@@ -328,7 +328,7 @@ static ListPlan plan_lists(const Plan &p, const Batch &b, int64_t most) {
         std::max<int64_t>(std::max<int64_t>(at / 4, known ? p.list_more : 0), int64_t(1) << 16),
         most / 4);
     lp.total = at + more;
-    lp.row_cap = !p.forces && b.natoms > kMarkAtoms ? lp.total * 4 / kRowMark + 16 : 0;
+    lp.row_cap = known && b.natoms > kMarkAtoms ? lp.total * 4 / kRowMark + 16 : 0;
     return lp;
 }
 int64_t ListPlan::cap(const Batch &b, size_t s) const {

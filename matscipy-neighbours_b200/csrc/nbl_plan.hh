@@ -102,8 +102,9 @@ struct Workspace {
 constexpr int kAutoWaves = 2;
 
 // Atoms above which the row of every 128th output slot is marked after the scan
-// (k_row_marks); below it, and beyond the marks' table, which has room for as many
-// pairs as the lists, the fill's warps search the row offsets.  Measured, fill and marks
+// (k_row_marks), from the second count of the same sizes on; below it, and beyond the
+// marks' table, which has room for as many pairs as the lists, the fill's warps search
+// the row offsets.  Measured, fill and marks
 // with / without, us, uniform gases: a million atoms at 10 / 2 / 0.5 per cell 704 / 713,
 // 183 / 182, 74 / 73; 200,000 130 / 133, 37 / 38, 22 / 20; 131,072 81 / 86, 29 / 29,
 // 16 / 15; 30,000 30 / 30, 11 / 10, 11 / 10: a launch for little, paid back by long

@@ -485,8 +485,9 @@ def run_device(quantities, origin, cell, inv, pbc8, pos_t, host_pos, rc, per_ato
                        per_type_sq, ncut, types, device_id)
     sp = ctypes.c_void_p(stream.cuda_stream)
 
+    npairs = ctypes.c_int64()
+
     def count():
-        npairs = ctypes.c_int64()
         if atom_range is not None:
             check(lib.nbl_set_atom_range(plan, int(atom_range[0]), int(atom_range[1])))
         try:
@@ -496,13 +497,13 @@ def run_device(quantities, origin, cell, inv, pbc8, pos_t, host_pos, rc, per_ato
                 # The range applies to the count just made (and its fill);
                 # later calls on this thread's plan build full lists again.
                 lib.nbl_set_atom_range(plan, 0, -1)
-        return int(npairs.value)
+        return npairs.value
 
     ctx = torch.cuda.device(dev) if torch.cuda.current_device() != device_id else _NO_CONTEXT
     with ctx:
         bufs = with_room(plan, torch.OutOfMemoryError, count,
                          lambda n: _device_outputs(torch, quantities, n, dev))
-        if any(t.shape[0] for t in bufs.values()):
+        if npairs.value:
             o = _outputs_struct(bufs, lambda t: t.data_ptr())
             check(lib.nbl_fill(plan, ctypes.byref(o), sp))
     return bufs

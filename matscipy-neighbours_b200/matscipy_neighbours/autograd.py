@@ -61,13 +61,18 @@ def _function():
 
             def count():
                 _ext.check(_ext.lib.nbl_count(plan, ctypes.byref(req), sp, ctypes.byref(n)))
-                return int(n.value)
+                return n.value
+
+            def outputs(P):
+                return (torch.empty(P, dtype=torch.int32, device=dev),
+                        torch.empty(P, dtype=torch.int32, device=dev),
+                        torch.empty((P, 3), dtype=torch.float64, device=dev),
+                        torch.empty(P, dtype=torch.float64, device=dev),
+                        torch.empty((P, 3), dtype=torch.int32, device=dev))
 
             with torch.cuda.device(dev):
-                bufs = _ext.with_room(plan, torch.OutOfMemoryError, count,
-                                      lambda P: _ext._device_outputs(torch, "ijDdS", P, dev))
-                i, j, D, d, S = (bufs[ch] for ch in "ijDdS")
-                P = int(n.value)
+                i, j, D, d, S = _ext.with_room(plan, torch.OutOfMemoryError, count, outputs)
+                P = n.value
                 off = None  # (the default backward reads no row offsets)
                 if deterministic:
                     off = torch.empty(nat + 1, dtype=torch.int64, device=dev)
