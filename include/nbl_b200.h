@@ -194,7 +194,8 @@ NBL_API nbl_status nbl_plan_set_launch(nbl_plan *plan, int count_ctas_per_sm, in
      thread_per_atom                      0 = the row passes, whose count takes
                                           one thread per atom where the
                                           occupied cells hold fewer than four
-                                          atoms on average (known after a first
+                                          atoms on average and no more pairs
+                                          than such cells give (known after a first
                                           count of the same sizes; before it
                                           empty cells count too), -1 = the warp
                                           passes, 1 = one thread per atom in

@@ -20,21 +20,22 @@
 // ballots, scans and tables) the passes are made of instructions around the
 // pairs, and rows written one by one leave a partial sector at both ends of
 // every row in each of five arrays.  Measured, count + fill: 200,000 atoms of a
-// slab with per-type cutoffs 84 + 25 us (187 + 120 one thread per atom writing
-// its own row), a gas of two neighbours per atom 62 + 23 (73 + 97); the fill
-// alone 612 us for the 48 M pairs of a million-atom metal (1,051 from hit words,
-// a warp per cell), 4.0 TB/s of output, bound by L1 wavefronts (75 %: position
+// slab with per-type cutoffs 85 + 21 us (187 + 120 one thread per atom writing
+// its own row), a gas of two neighbours per atom 61 + 20 (73 + 97); the fill
+// alone 616 us for the 48 M pairs of a million-atom metal (1,051 from hit words,
+// a warp per cell), 4.0 TB/s of output, bound by L1 wavefronts (79 %: position
 // gathers, staging) and the loads' latency.
 //
-// Which count: this one where the occupied cells hold fewer than kSparseAtoms
-// atoms on average, and with plain FP64 tests; k_count_list (nbl_trav_list.cu)
-// elsewhere.  On the slab (2.3 atoms per occupied cell) 84 against 214 us, on
-// the dense bulk (10 per cell) 674 against 490.
+// Which count: this one on sparse grids (kSparseAtoms, in nbl_plan.hh, with both
+// sides measured) and with plain FP64 tests; k_count_list (nbl_trav_list.cu)
+// elsewhere.
 //
-// Lists: atom i of a system owns list_cap 16-byte groups at list_base + i *
-// list_cap, the last one a link to a chunk of kListChunk more, whose last group
-// links on.  When the chunks run out the row keeps its length, kErrNoList is set, and the row
-// is written by the thread-per-atom fill instead (nbl_trav_atoms.cu).
+// Lists: atom i of a system, if its row is in range, owns list_cap 16-byte groups at
+// list_base + i * list_cap, the last one a link to a chunk of kListChunk more, whose
+// last group links on.  When the chunks run out the row keeps its length, asks for the
+// chunks it lacks all the same (a synchronised count is then made once more, with
+// that room), and kErrNoList is set; a row that still has no list is written by the
+// thread-per-atom fill (nbl_trav_atoms.cu).
 #include "nbl_stages.cuh"
 #include "nbl_traverse.cuh"
 

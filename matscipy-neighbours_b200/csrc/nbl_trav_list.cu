@@ -17,16 +17,16 @@
 // 32 candidates, hits compacted by population counts) the same pass took 611 us
 // on the dense bulk (1,048,576 atoms), bound by the population counts' slow
 // pipe; with one thread per atom 674 us, because a warp's atoms lie in three
-// cells whose candidates differ.  This form: 490 us there (the two-pass scheme
-// that wrote hit words took 371, but its fill 1,051 against 653 us from these
-// lists), 27 + 17 us for 10,007 atoms (36 + 36 before).  Bound by instruction
-// issue: about 180 us staging and set-up, 150 the sweep, 160 the entries.
+// cells whose candidates differ.  This form: 492 us there (the two-pass scheme
+// that wrote hit words took 371, but its fill 1,051 against 616 us from these
+// lists), 25 + 15 us for 10,007 atoms (36 + 36 before).  Bound by the latency of
+// staging and list writes at 17 warps per SM, 0.5 instructions a cycle: about 180 us
+// staging and set-up, 150 the sweep, 160 the entries.
 //
-// Where an atom visits many candidates (CULL: more than two full tables on
-// average, small cells with cutoffs beyond them) the ones outside the tile's
-// bounding box plus the cutoff never reach the table: 1,550 against 2,411 us on
-// 4,096 small periodic systems of about 3,000 candidates per atom.  Below that
-// the test costs more than it saves (527 against 490 us on the dense bulk).
+// Where an atom visits many candidates (CULL: more than one full table on average,
+// kCullCand) the ones outside the tile's bounding box plus the cutoff never reach the
+// table: 1,443 us on 4,096 small periodic systems of about 3,000 candidates per atom
+// (2,411 without, at four CTAs per SM).
 #include "nbl_traverse.cuh"
 
 namespace nbl {
