@@ -814,6 +814,7 @@ static void gather_args(const Plan &p, const Batch &b, const uint32_t *skeys,
     ga.items = nullptr;
     ga.n_items = B.small + 3;
     ga.itile = 0;
+    ga.crowd = INT32_MAX;
 }
 
 static void traverse_args(Plan &p, const Batch &b, bool atoms, int max_run) {
@@ -908,6 +909,8 @@ static nbl_status enqueue_build(Plan &p, const Batch &b, bool atoms, int max_run
             if (items && max_run == 1) {  // one cell per item: the gather makes them
                 ga.items = B.items;
                 ga.itile = tile_of(p, b);
+                ga.crowd = (int)std::min<int64_t>(std::max<int64_t>(64 * N / b.table_size, 256),
+                                                  INT32_MAX);
                 ga.home = nullptr;
             }
         } else {

@@ -221,7 +221,8 @@ __device__ __forceinline__ void gather_one(const GatherArgs &a, int64_t s) {
             a.home[base + __popc(m & lanemask_lt())] = h;
         }
         if (a.items != nullptr) {  // the cell's work items (tiles_one, one cell each)
-            const int nt = start ? (seg.y - seg.x + a.itile - 1) / a.itile : 0;
+            const int tile = seg.y - seg.x > a.crowd ? min(a.itile, kCrowdTile) : a.itile;
+            const int nt = start ? (seg.y - seg.x + tile - 1) / tile : 0;
             int incl = nt;
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
@@ -237,8 +238,8 @@ __device__ __forceinline__ void gather_one(const GatherArgs &a, int64_t s) {
                 w.c[1] = c[1];
                 w.c[2] = c[2];
                 w.sys = sysid;
-                w.ib = seg.x + a.itile * t;
-                w.nt = min(a.itile, seg.y - w.ib);
+                w.ib = seg.x + tile * t;
+                w.nt = min(tile, seg.y - w.ib);
                 w.tidx = (int32_t)tidx;
                 w.run = 1;
                 a.items[first + t] = w;
