@@ -376,28 +376,25 @@ def _parse(quantities, cell_origin, cell, inv_cell, pbc, positions, cutoffs, typ
     return origin, cell, inv, pbc8, ty
 
 
-def with_room(plan, errors, count, then):
-    """``then(count())``.  The count leaves neighbour lists in the plan's workspace, about
-    a sixth of what the outputs take: where the device has no room for those beside the
-    lists (one of `errors`), the workspace is given back and the pairs are counted again
-    by hit words (thread_per_atom = -1), which take a tenth of the lists."""
-    n = count()
-    try:
-        return then(n)
-    except errors:
-        cfg = LaunchConfig()
-        check(lib.nbl_plan_get_launch_config(plan, ctypes.byref(cfg)))
-        if cfg.thread_per_atom != 0 or cfg.cells_per_item != 0:
-            raise   # no lists
-    # (out of the handler: the exception held what `then` had allocated)
+def count_without_lists(plan, count):
+    """Counts again by hit words.  The count leaves neighbour lists in the plan's
+    workspace, about a sixth of what the outputs take: where the device had no room for
+    those beside the lists, the workspace is given back and `count` called with the hit
+    words (thread_per_atom = -1), which take a tenth of the lists.  False if the count
+    had no lists."""
+    cfg = LaunchConfig()
+    check(lib.nbl_plan_get_launch_config(plan, ctypes.byref(cfg)))
+    if cfg.thread_per_atom != 0 or cfg.cells_per_item != 0:
+        return False
     cfg.thread_per_atom = -1
     check(lib.nbl_plan_set_launch_config(plan, ctypes.byref(cfg)))
     try:
         check(lib.nbl_plan_trim(plan))
-        return then(count())
+        count()
     finally:
         cfg.thread_per_atom = 0
         lib.nbl_plan_set_launch_config(plan, ctypes.byref(cfg))
+    return True
 
 
 def run_host(quantities, origin, cell, inv, pbc8, pos, rc, per_atom, per_type_sq,
@@ -409,20 +406,20 @@ def run_host(quantities, origin, cell, inv, pbc8, pos, rc, per_atom, per_type_sq
     req = make_request(flags, origin, cell, inv, pbc8, nat,
                        ctypes.c_void_p(pos.ctypes.data) if nat else None, False, rc,
                        per_atom, per_type_sq, ncut, types, device_id)
+    npairs = ctypes.c_int64()
 
     def count():
-        npairs = ctypes.c_int64()
         check(lib.nbl_count(plan, ctypes.byref(req), None, ctypes.byref(npairs)))
-        return int(npairs.value)
 
-    def fill(n):
-        bufs = _host_outputs(quantities, n)
-        if n:
-            o = _outputs_struct(bufs, lambda a: a.ctypes.data)
-            check(lib.nbl_fill_host(plan, ctypes.byref(o), None))
-        return bufs
-
-    return with_room(plan, MemoryError, count, fill)
+    count()
+    bufs = _host_outputs(quantities, npairs.value)
+    if npairs.value:
+        o = _outputs_struct(bufs, lambda a: a.ctypes.data)
+        st = lib.nbl_fill_host(plan, ctypes.byref(o), None)
+        if st == NBL_ERROR_OUT_OF_MEMORY and count_without_lists(plan, count):
+            st = lib.nbl_fill_host(plan, ctypes.byref(o), None)
+        check(st)
+    return bufs
 
 
 def neighbour_list(quantities, cell_origin, cell, inv_cell, pbc, positions, cutoffs,
@@ -497,12 +494,18 @@ def run_device(quantities, origin, cell, inv, pbc8, pos_t, host_pos, rc, per_ato
                 # The range applies to the count just made (and its fill);
                 # later calls on this thread's plan build full lists again.
                 lib.nbl_set_atom_range(plan, 0, -1)
-        return npairs.value
 
     ctx = torch.cuda.device(dev) if torch.cuda.current_device() != device_id else _NO_CONTEXT
     with ctx:
-        bufs = with_room(plan, torch.OutOfMemoryError, count,
-                         lambda n: _device_outputs(torch, quantities, n, dev))
+        count()
+        bufs = None
+        try:
+            bufs = _device_outputs(torch, quantities, npairs.value, dev)
+        except torch.OutOfMemoryError:
+            if not count_without_lists(plan, count):
+                raise
+        if bufs is None:  # (out of the handler, which holds what was allocated)
+            bufs = _device_outputs(torch, quantities, npairs.value, dev)
         if npairs.value:
             o = _outputs_struct(bufs, lambda t: t.data_ptr())
             check(lib.nbl_fill(plan, ctypes.byref(o), sp))
@@ -650,15 +653,23 @@ def neighbour_matrix_tensors(cell_origin, cell, inv_cell, pbc, host_pos, cutoffs
     overflow = ctypes.c_int(0)
     ctx = torch.cuda.device(dev) if torch.cuda.current_device() != dev_id else _NO_CONTEXT
     with ctx:
-        # (the fill writes every slot, the unused ones with zeros)
-        idx, dist, count = with_room(
-            plan, torch.OutOfMemoryError,
-            lambda: check(lib.nbl_count(plan, ctypes.byref(req),
-                                        ctypes.c_void_p(stream.cuda_stream),
-                                        ctypes.byref(npairs))),
-            lambda _: (torch.empty((nat, K), dtype=torch.int32, device=dev),
-                       torch.empty((nat, K, 3), dtype=torch.float64, device=dev),
-                       torch.empty((nat,), dtype=torch.int32, device=dev)))
+        def count_pairs():
+            check(lib.nbl_count(plan, ctypes.byref(req), ctypes.c_void_p(stream.cuda_stream),
+                                ctypes.byref(npairs)))
+
+        def outputs():  # (the fill writes every slot, the unused ones with zeros)
+            return (torch.empty((nat, K), dtype=torch.int32, device=dev),
+                    torch.empty((nat, K, 3), dtype=torch.float64, device=dev),
+                    torch.empty((nat,), dtype=torch.int32, device=dev))
+
+        count_pairs()
+        outs = None
+        try:
+            outs = outputs()
+        except torch.OutOfMemoryError:
+            if not count_without_lists(plan, count_pairs):
+                raise
+        idx, dist, count = outs or outputs()
         if nat:
             check(lib.nbl_fill_matrix(plan, K, ctypes.c_void_p(idx.data_ptr()),
                                       ctypes.c_void_p(dist.data_ptr()),

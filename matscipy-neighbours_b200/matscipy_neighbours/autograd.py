@@ -61,7 +61,6 @@ def _function():
 
             def count():
                 _ext.check(_ext.lib.nbl_count(plan, ctypes.byref(req), sp, ctypes.byref(n)))
-                return n.value
 
             def outputs(P):
                 return (torch.empty(P, dtype=torch.int32, device=dev),
@@ -71,8 +70,15 @@ def _function():
                         torch.empty((P, 3), dtype=torch.int32, device=dev))
 
             with torch.cuda.device(dev):
-                i, j, D, d, S = _ext.with_room(plan, torch.OutOfMemoryError, count, outputs)
+                count()
+                outs = None
+                try:
+                    outs = outputs(n.value)
+                except torch.OutOfMemoryError:
+                    if not _ext.count_without_lists(plan, count):
+                        raise
                 P = n.value
+                i, j, D, d, S = outs or outputs(P)
                 off = None  # (the default backward reads no row offsets)
                 if deterministic:
                     off = torch.empty(nat + 1, dtype=torch.int64, device=dev)
